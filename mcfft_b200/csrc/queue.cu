@@ -12,6 +12,7 @@ namespace mcfft {
 
 int queue_variant(const TileKernel& k) {
   const int L = k.L;
+  if (k.reg_kind >= 0) return -1;
   if (L < 32 || L > 4096 || (L & (L - 1))) return -1;
   if (k.split) {
     if (k.tile_points != 8192 || L > 2048) return -1;

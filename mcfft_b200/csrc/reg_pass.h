@@ -1,0 +1,45 @@
+// reg_pass.h -- host side of the register pass kernels (fft_reg.cuh):
+// variant entries, staging descriptions and twiddle tables.
+#pragma once
+#include "fft_reg.cuh"
+#include "tile_pass.h"
+
+namespace mcfft {
+
+// Variants by form, each in a translation unit of its own.
+const std::vector<TileKernel>& reg_registry_plain();    // reg_plain.cu
+const std::vector<TileKernel>& reg_registry_split();    // reg_split.cu
+const std::vector<TileKernel>& reg_registry_split16();  // reg_split16.cu
+
+// Register kernel of a pass with points along `ik` in and `ok` out, or null.
+const TileKernel* find_reg_kernel(int L, layout::Kind ik, layout::Kind ok, bool posttw, bool split,
+                                  int tile_points, bool in16);
+
+// Where TMA places a tile of the variant in shared memory (RegPass::load1_*
+// and store2_*), for a pass with the given strides (elements).
+void reg_stagings(const TileKernel& k, layout::Kind ik, layout::Kind ok, int in_elem, int out_elem,
+                  int64_t in_sp, int64_t in_sc, int64_t in_so, int64_t out_sp, int64_t out_sc,
+                  int64_t out_so, int64_t ncols, int64_t nouter, layout::Staging* in,
+                  layout::Staging* out);
+
+// Phase-1 twiddles W_L^(k v) * scale in the layout of RegPass (mode 0: FP32,
+// 8 bytes at k NV + v; 1: doubled for two columns, 16 bytes; 2: pairs (2i,
+// 2i + 1), 16 bytes at i NV + v); sign -1 forward, +1 inverse.
+cudaError_t gen_reg_twiddles(void* dst, int L, int NV, int mode, int sign, double scale,
+                             cudaStream_t st);
+
+template <int L, int R1, int R2, int TP, bool IN16, bool OUT16, int KIND, bool POST>
+TileKernel make_reg() {
+  using P = reg::RegPass<L, R1, R2, TP, IN16, OUT16, KIND, POST, false>;
+  using Q = reg::RegPass<L, R1, R2, TP, IN16, OUT16, KIND, POST, true>;
+  TileKernel k{reinterpret_cast<const void*>(&reg::fft_reg<P>), L, R1, P::C, POST, !OUT16, P::THREADS,
+               P::SMEM_BYTES, 0, TP, IN16};
+  k.fn_inv = reinterpret_cast<const void*>(&reg::fft_reg<Q>);
+  k.reg_kind = KIND;
+  k.reg_h = P::h;
+  k.tw_bytes = P::TWB;
+  k.tw_mode = P::PK ? (R1 == 32 ? 2 : 1) : 0;
+  return k;
+}
+
+}  // namespace mcfft

@@ -177,6 +177,7 @@ cudaError_t launch_tile_pass(const TilePass& tp, const void* in, void* out, int 
   a.bmat = tp.bmat[dir];
   a.bmat_lo = tp.bmat_lo[dir];
   a.inverse = dir;
+  const void* fn = tp.k->fn_of(dir);
   // The shared-memory limit is a per-device attribute of the function.
   static std::mutex mu;
   static std::vector<std::pair<int, const void*>> configured;
@@ -185,12 +186,12 @@ cudaError_t launch_tile_pass(const TilePass& tp, const void* in, void* out, int 
     if (cudaGetDevice(&dev) != cudaSuccess) return cudaGetLastError();
     std::lock_guard<std::mutex> lock(mu);
     bool done = false;
-    for (const auto& f : configured) done |= (f.first == dev && f.second == tp.k->fn);
+    for (const auto& f : configured) done |= (f.first == dev && f.second == fn);
     if (!done) {
-      cudaError_t e = cudaFuncSetAttribute(tp.k->fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            tp.k->smem_bytes);
       if (e != cudaSuccess) return e;
-      configured.push_back({dev, tp.k->fn});
+      configured.push_back({dev, fn});
     }
   }
   void* args[] = {&a};
@@ -204,7 +205,7 @@ cudaError_t launch_tile_pass(const TilePass& tp, const void* in, void* out, int 
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = pdl ? 1 : 0;
-  return cudaLaunchKernelExC(&cfg, tp.k->fn, args);
+  return cudaLaunchKernelExC(&cfg, fn, args);
 }
 
 void fill_tile_args(TilePass* tp) {

@@ -19,6 +19,15 @@ struct TileKernel {
   int tmem_cols;
   int tile_points;
   bool in16;  // split form: FP16 input staging (FP32 otherwise); plain: always
+  // Register kernels (reg_pass.h; `fn` is then the forward direction's, R the
+  // first radix): RegKind (-1: a tcgen05 kernel, one function for both
+  // directions), the inverse direction's function, and the shape of the
+  // staging and of the twiddle table.
+  int reg_kind = -1;
+  const void* fn_inv = nullptr;
+  int reg_h = 0;
+  int tw_bytes = 0, tw_mode = 0;
+  const void* fn_of(int dir) const { return dir && fn_inv ? fn_inv : fn; }
 };
 
 // Split-form variants (tile_split.cu).

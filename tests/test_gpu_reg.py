@@ -1,0 +1,77 @@
+"""Register pass kernels on the GPU: every length they hold in each form and
+direction, with enough tiles that every CTA reuses its buffers many times
+(both groups of the split form), a ragged last tile, passes with fewer columns
+than a tile, and four-step pairs over many transforms.  A sample of the
+transforms is compared with the FP64 oracle; bounds as in test_gpu_parity."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+if not torch.cuda.is_available():
+    pytest.skip("needs a GPU", allow_module_level=True)
+pytestmark = pytest.mark.gpu
+
+import mcfft_b200 as mc  # noqa: E402
+from oracle import oracle  # noqa: E402
+from tests.gpu_util import compare, from_device, rounded, to_device  # noqa: E402
+
+FORMS = {"plain": (mc.PREC_FP16, 0, True, 1e-3), "split": (mc.PREC_SPLIT, 0, False, 2e-6),
+         "split16": (mc.PREC_SPLIT, mc.FLAG_INPUT_F16, True, 2e-6)}
+
+
+def _check(shape, batch, form, direction):
+    prec, flags, f16, tol = FORMS[form]
+    n = int(np.prod(shape))
+    rng = np.random.default_rng(n + batch)
+    # a few distinct transforms, repeated over the batch
+    kinds = min(batch, 5)
+    x = rng.uniform(-1, 1, (kinds, n)) + 1j * rng.uniform(-1, 1, (kinds, n))
+    xd = to_device(x, f16).reshape(kinds, n)
+    pick = torch.arange(batch, device="cuda") % kinds
+    if f16:
+        xs = torch.view_as_real(xd)[pick].contiguous()
+        xs = torch.view_as_complex(xs)
+    else:
+        xs = xd[pick].contiguous()
+    odt = torch.complex64 if prec == mc.PREC_SPLIT else torch.complex32
+    out = torch.empty(batch * n, dtype=odt, device="cuda")
+    out.view(torch.uint8).fill_(0xFF)
+    with mc.Plan(shape, batch, prec, flags) as p:
+        p.exec_ptr(xs.data_ptr(), out.data_ptr(), direction, torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        p.check_status()
+        scale = 2.0 ** p.info().scale_log2
+    # every transform equals the first one of its kind, bit for bit
+    words = out.view(torch.int32).reshape(batch, -1)
+    for k in range(kinds):
+        same = (words[k::kinds] == words[k]).all()
+        assert bool(same), f"transforms of one input differ (kind {k})"
+    xr = rounded(x, f16).reshape((kinds,) + tuple(shape))
+    if direction == mc.FORWARD:
+        ref = oracle.fftnd(xr, list(shape)) * scale
+    else:
+        ref = np.conj(oracle.fftnd(np.conj(xr), list(shape))) * scale
+    y = from_device(out[:kinds * n])
+    rel, mx = compare(y, ref)
+    assert rel < tol, (rel, mx)
+
+
+@pytest.mark.parametrize("direction", [mc.FORWARD, mc.INVERSE])
+@pytest.mark.parametrize("form", list(FORMS))
+@pytest.mark.parametrize("n", [64, 128, 256, 512, 1024])
+def test_rows(n, form, direction):
+    _check((n,), (9 << 20) // n + 3, form, direction)
+
+
+@pytest.mark.parametrize("direction", [mc.FORWARD, mc.INVERSE])
+@pytest.mark.parametrize("form", list(FORMS))
+@pytest.mark.parametrize("n,batch", [(1 << 14, 301), (1 << 17, 61), (1 << 18, 30), (1 << 20, 9)])
+def test_four_step(n, batch, form, direction):
+    _check((n,), batch, form, direction)
+
+
+@pytest.mark.parametrize("form", list(FORMS))
+@pytest.mark.parametrize("shape,batch", [((64, 32), 3), ((128, 16), 5), ((256, 32), 9), ((512, 16), 3),
+                                         ((1024, 64), 150), ((64, 128, 32), 7), ((256, 64, 16), 11)])
+def test_columns(shape, batch, form):
+    _check(shape, batch, form, mc.FORWARD)
