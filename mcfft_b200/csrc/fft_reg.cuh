@@ -80,6 +80,29 @@ __device__ __forceinline__ uint32_t lds32(uint32_t addr) {
   return v;
 }
 
+// Bounded wait; after a timeout (here or elsewhere in the block) it returns
+// at once, leaving the abort flag set.
+__device__ __forceinline__ void wait_or_abort(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+  if (sm100::mbar_try_wait(bar, parity)) return;
+  const uint32_t t0 = sm100::globaltimer_ns();
+  while (!sm100::mbar_try_wait(bar, parity)) {
+    if (*abort_flag) return;
+    if (sm100::globaltimer_ns() - t0 > kWaitLimit) {
+      *abort_flag = 1;
+      return;
+    }
+  }
+}
+
+// Barrier among the T threads of a group.
+template <int T>
+struct Sync {
+  int bar;
+  __device__ __forceinline__ void group() const {
+    asm volatile("bar.sync %0, %1;" ::"r"(bar), "n"(T) : "memory");
+  }
+};
+
 template <int L_, int R1_, int R2_, int TP_, bool IN16_, bool OUT16_, int KIND_, bool POST_, bool INV_>
 struct RegPass {
   static constexpr int L = L_, R1 = R1_, R2 = R2_, TP = TP_, KIND = KIND_;
@@ -112,7 +135,7 @@ struct RegPass {
   // of the other's tile in the same buffer, and a parity wait is only right
   // for a waiter that has seen the phase before.
   static constexpr int NFULL = NG == 1 ? NBUF : NG * NBUF;
-  static constexpr int THREADS = NG * T + 32;
+  static constexpr int THREADS = NG * T + 128;
   static constexpr int OFF_TW = NBUF * BUF;
   static constexpr int OFF_BAR = OFF_TW + TWB;
   static constexpr int SMEM_BYTES = OFF_BAR + 128 + 1024;
@@ -280,24 +303,27 @@ struct RegPass {
     return make_float2(cs, INV ? sn : -sn);
   }
 
-  struct Sync {
-    int bar;  // named barrier of this group
-    __device__ __forceinline__ void group() const {
-      asm volatile("bar.sync %0, %1;" ::"r"(bar), "n"(T) : "memory");
-    }
+  // Tables that depend on the plan (none here).
+  template <class A>
+  static __device__ __forceinline__ void setup(const A&, uint8_t*, int) {}
+
+  // What a thread keeps for the whole launch (nothing here).
+  struct State {
+    template <class A>
+    __device__ __forceinline__ State(const A&, int) {}
   };
 
   // One tile in buffer sb; t: thread of the group, tws: twiddle table.
   template <class A>
-  static __device__ __forceinline__ void run(const A& a, uint32_t sb, uint32_t tws, int t, uint32_t cb,
-                                             const Sync& sync) {
+  static __device__ __forceinline__ void run(const A& a, const State&, uint32_t sb, uint32_t tws, int t, uint32_t cb,
+                                             const Sync<T>& sync) {
     if constexpr (PK) run_pk(a, sb, tws, t, cb, sync);
     else run_f32(a, sb, tws, t, cb, sync);
   }
 
   template <class A>
   static __device__ __forceinline__ void run_pk(const A& a, uint32_t sb, uint32_t tws, int t, uint32_t cb,
-                                                const Sync& sync) {
+                                                const Sync<T>& sync) {
     P2 re[16], im[16];
     {  // ------------------------------------------------------- phase 1
       uint32_t w[V1][R1], b[V1], v = 0, c = 0;
@@ -425,7 +451,7 @@ struct RegPass {
 
   template <class A>
   static __device__ __forceinline__ void run_f32(const A& a, uint32_t sb, uint32_t tws, int t, uint32_t cb,
-                                                 const Sync& sync) {
+                                                 const Sync<T>& sync) {
     {  // ------------------------------------------------------- phase 1
       float re[V1][R1], im[V1][R1];
       uint32_t v[V1], c[V1];
@@ -531,20 +557,6 @@ struct RegPass {
   }
 };
 
-// Bounded wait; after a timeout (here or elsewhere in the block) it returns
-// at once, leaving the abort flag set.
-__device__ __forceinline__ void wait_or_abort(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
-  if (sm100::mbar_try_wait(bar, parity)) return;
-  const uint32_t t0 = sm100::globaltimer_ns();
-  while (!sm100::mbar_try_wait(bar, parity)) {
-    if (*abort_flag) return;
-    if (sm100::globaltimer_ns() - t0 > kWaitLimit) {
-      *abort_flag = 1;
-      return;
-    }
-  }
-}
-
 template <class P>
 __global__ void __launch_bounds__(P::THREADS, 1) fft_reg(const __grid_constant__ TileArgs a) {
   constexpr int NG = P::NG, T = P::T, NW = P::NW, NBUF = P::NBUF;
@@ -567,9 +579,10 @@ __global__ void __launch_bounds__(P::THREADS, 1) fft_reg(const __grid_constant__
       tile::prefetch_tmap(&a.tmap_in);
       tile::prefetch_tmap(&a.tmap_out);
     }
-  } else {
+  } else if (warp < NG * NW) {
     for (int i = tid; i < P::TWB / 16; i += NG * T)
       *reinterpret_cast<float4*>(smem + P::OFF_TW + 16 * i) = __ldg(a.tw + i);
+    P::setup(a, smem + P::OFF_TW, tid);
   }
   __syncthreads();
   // Up to here only this launch's constant tables were read; the buffers the
@@ -579,8 +592,9 @@ __global__ void __launch_bounds__(P::THREADS, 1) fft_reg(const __grid_constant__
   // 32-bit tile arithmetic (the plan refuses more tiles than that)
   const uint32_t step = gridDim.x, ntiles = (uint32_t)a.ntiles, ncb = (uint32_t)a.col_blocks;
   const uint32_t mine = ntiles > blockIdx.x ? (ntiles - 1 - blockIdx.x) / step + 1 : 0;
-  if (producer) {
-    if (lane == 0) {
+  if (warp >= NG * NW) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 24;");
+    if (producer && lane == 0) {
       auto load = [&](uint32_t i) {
         const uint32_t t = blockIdx.x + i * step, b = i % NBUF;
         int32_t crd[5];
@@ -610,12 +624,14 @@ __global__ void __launch_bounds__(P::THREADS, 1) fft_reg(const __grid_constant__
     }
     __syncwarp();
   } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
     const int grp = NG == 1 ? 0 : tid / T, t = tid - grp * T;
-    const typename P::Sync sync{1 + grp};
+    const Sync<T> sync{1 + grp};
+    const typename P::State st(a, t);
     for (uint32_t i = grp; i < mine; i += NG) {
       const uint32_t b = i % NBUF;
       wait_or_abort(&full[i % NFULL], (i / NFULL) & 1u, abort_flag);
-      P::run(a, base_u + b * P::BUF, base_u + P::OFF_TW, t, (blockIdx.x + i * step) % ncb, sync);
+      P::run(a, st, base_u + b * P::BUF, base_u + P::OFF_TW, t, (blockIdx.x + i * step) % ncb, sync);
       sm100::fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) tile::mbar_arrive(&done[b]);

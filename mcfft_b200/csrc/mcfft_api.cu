@@ -479,8 +479,17 @@ mcfftResult add_tile_pass(mcfftPlan p, const PassSpec& s, int only_tile_points =
   if (k->reg_kind >= 0) {
     for (int dir = 0; dir < 2; ++dir) {
       float4* tw = nullptr;
-      r = plan_alloc(p, &tw, (size_t)k->tw_bytes);
+      r = plan_alloc(p, &tw, (size_t)k->tw_bytes + (k->mma ? 2048 : 0));
       if (r) return r;
+      if (k->mma) {  // twiddle table, then the matrix fragments
+        std::vector<uint32_t> tab((size_t)k->tw_bytes / 4 + 512);
+        k->fill_tw[dir](reinterpret_cast<float*>(tab.data()));
+        k->fill_frag[dir](tab.data() + k->tw_bytes / 4);
+        const cudaError_t e = cudaMemcpy(tw, tab.data(), tab.size() * 4, cudaMemcpyHostToDevice);
+        if (e != cudaSuccess) return cuda_fail(e);
+        tp.tw[dir] = tw;
+        continue;
+      }
       const cudaError_t e = gen_reg_twiddles(tw, k->L, k->L / k->R, k->tw_mode, dir == 0 ? -1 : 1,
                                              p->split ? 1.0 : 1.0 / k->R, 0);
       if (e != cudaSuccess) return cuda_fail(e);
@@ -533,7 +542,7 @@ mcfftResult add_tile_pass(mcfftPlan p, const PassSpec& s, int only_tile_points =
     a.post_scale = tables ? 0.f : (float)(2.0 / (double)s.postN);
   }
   for (int dir = 0; dir < 2; ++dir) {
-    tp.bmat[dir] = p->bsw64[dir];
+    tp.bmat[dir] = k->mma ? reinterpret_cast<const uint4*>(tp.tw[dir] + k->tw_bytes / 16) : p->bsw64[dir];
     tp.bmat_lo[dir] = p->bsw64_lo[dir];
   }
   int occ = 1;

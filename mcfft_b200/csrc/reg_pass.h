@@ -1,6 +1,7 @@
 // reg_pass.h -- host side of the register pass kernels (fft_reg.cuh):
 // variant entries, staging descriptions and twiddle tables.
 #pragma once
+#include "fft_mma.cuh"
 #include "fft_reg.cuh"
 #include "tile_pass.h"
 
@@ -39,6 +40,23 @@ TileKernel make_reg() {
   k.reg_h = P::h;
   k.tw_bytes = P::TWB;
   k.tw_mode = P::PK ? (R1 == 32 ? 2 : 1) : 0;
+  return k;
+}
+
+template <int L, int KIND, bool POST>
+TileKernel make_mma() {
+  using P = reg::MmaPass<L, KIND, POST, false>;
+  using Q = reg::MmaPass<L, KIND, POST, true>;
+  TileKernel k{reinterpret_cast<const void*>(&reg::fft_reg<P>), L, P::R, P::C, POST, false, P::THREADS,
+               P::SMEM_BYTES, 0, P::TP, true};
+  k.fn_inv = reinterpret_cast<const void*>(&reg::fft_reg<Q>);
+  k.reg_kind = KIND;
+  k.tw_bytes = P::TWB;
+  k.mma = true;
+  k.fill_tw[0] = &P::fill_twiddles;
+  k.fill_tw[1] = &Q::fill_twiddles;
+  k.fill_frag[0] = &P::fill_fragments;
+  k.fill_frag[1] = &Q::fill_fragments;
   return k;
 }
 

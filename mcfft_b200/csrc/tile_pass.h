@@ -27,6 +27,11 @@ struct TileKernel {
   const void* fn_inv = nullptr;
   int reg_h = 0;
   int tw_bytes = 0, tw_mode = 0;
+  // Tensor-core register kernels (fft_mma.cuh): host functions that fill the
+  // twiddle table and the matrix fragments of each direction.
+  bool mma = false;
+  void (*fill_tw[2])(float*) = {nullptr, nullptr};
+  void (*fill_frag[2])(uint32_t*) = {nullptr, nullptr};
   const void* fn_of(int dir) const { return dir && fn_inv ? fn_inv : fn; }
 };
 

@@ -3,12 +3,15 @@
 // put it, the exchange hands phase 2 the vectors phase 1 wrote, every store
 // lands where the TMA store expects it, all accesses stay inside the buffer,
 // what is written in place belongs to the warp that read it, and no access
-// has bank conflicts.  Prints one line per variant; exit status 1 on a fault.
+// has bank conflicts.  Where TMA puts or takes a point is worked out from the
+// tensor-map dimensions, not from the kernels' own formulas.  Prints one line
+// per variant; exit status 1 on a fault.
 #include <cstdio>
 #include <set>
 #include <vector>
 
-#include "../mcfft_b200/csrc/fft_reg.cuh"
+#include "../mcfft_b200/csrc/fft_mma.cuh"
+#include "../mcfft_b200/csrc/reg_staging.h"
 
 using namespace mcfft;
 using namespace mcfft::reg;
@@ -45,19 +48,42 @@ static int wavefronts(const std::vector<uint32_t>& a, int bytes) {
   return total;
 }
 
+// Byte of (pos, c) in shared memory as the tensor map's box places it (the box
+// of tile 0 over a pass of C columns): index pos * C + c.
+static std::vector<uint32_t> tma_place(const layout::Staging& s, bool row) {
+  std::vector<uint32_t> at((size_t)s.L * s.C, ~0u);
+  uint64_t n = 1;
+  for (int d = 0; d < s.ndims; ++d) n *= s.box[d];
+  CHECK(s.ndims >= 3 && s.ndims <= 5 && n == at.size(), "box of %llu points", (unsigned long long)n);
+  for (uint64_t i = 0; i < n; ++i) {
+    uint64_t r = i, g = 0;
+    for (int d = 0; d < s.ndims; ++d) {
+      const uint64_t x = r % s.box[d];
+      r /= s.box[d];
+      CHECK(s.box[d] <= 256, "box dimension %u", s.box[d]);
+      g += x * (d ? s.gstride_bytes[d] / s.elem : 1);
+    }
+    const uint64_t pos = row ? g % s.L : g / s.C, c = row ? g / s.L : g % s.C;
+    CHECK(pos < (uint64_t)s.L && c < (uint64_t)s.C, "element %llu", (unsigned long long)g);
+    uint32_t off = (uint32_t)(i * s.elem);
+    off ^= ((off >> 7) & s.swz) << 4;
+    if (pos < (uint64_t)s.L && c < (uint64_t)s.C) at[pos * s.C + c] = off;
+  }
+  for (uint32_t a : at) CHECK(a != ~0u, "a point outside the box");
+  return at;
+}
+
 template <class P>
 void check(const char* name) {
   const int bad0 = g_bad;
   const uint32_t in_bytes = P::TP * P::EI, mid_bytes = P::TP * P::EO;
-  auto in_at = [](uint32_t pos, uint32_t c) {
-    return P::KIND == kCC ? pos * P::RBI + c * P::EI : P::template row_base<P::EI>(pos, c);
-  };
-  auto out_at = [](uint32_t pos, uint32_t c) -> uint32_t {
-    if (P::KIND == kRR) return P::template row_base<P::EO>(pos, c);
-    if (P::KIND == kRC) return pos * P::RB + c * P::EO;
-    const uint32_t k1 = pos % P::R1, k2 = pos / P::R1;  // rows [k1 high][k2][k1 low]
-    return (((k1 >> P::h) * P::R2 + k2) * (1u << P::h) + (k1 & P::m)) * P::RB + c * P::EO;
-  };
+  const RegShape sh{P::L, P::R1, P::C, P::h, false};
+  const layout::Kind ik = P::KIND == kCC ? layout::COL : layout::ROW, ok = P::KIND == kRR ? layout::ROW : layout::COL;
+  const bool ri = ik == layout::ROW, ro = ok == layout::ROW;
+  const auto tin = tma_place(reg_staging_in(sh, ik, P::EI, ri ? 1 : P::C, ri ? P::L : 1, 0, P::C, 1), ri);
+  const auto tout = tma_place(reg_staging_out(sh, ik, ok, P::EO, ro ? 1 : P::C, ro ? P::L : 1, 0, P::C, 1), ro);
+  auto in_at = [&](uint32_t pos, uint32_t c) { return tin[pos * P::C + c]; };
+  auto out_at = [&](uint32_t pos, uint32_t c) { return tout[pos * P::C + c]; };
   int excess = 0;
   std::vector<int> seen(P::TP, 0);
   // slot -> (k1, v, c) after phase 1
@@ -143,12 +169,149 @@ void check(const char* name) {
   printf("%s %s (excess wavefronts %d)\n", g_bad == bad0 ? "ok" : "FAULT", name, excess);
 }
 
+template <class M>
+void check_mma(const char* name) {
+  const int bad0 = g_bad;
+  const uint32_t bytes = M::TP * 4;
+  const RegShape sh{M::L, M::R, M::C, 0, true};
+  const layout::Kind ik = M::KIND == kCC ? layout::COL : layout::ROW, ok = M::KIND == kRR ? layout::ROW : layout::COL;
+  const bool ri = ik == layout::ROW, ro = ok == layout::ROW;
+  const auto tin = tma_place(reg_staging_in(sh, ik, 4, ri ? 1 : M::C, ri ? M::L : 1, 0, M::C, 1), ri);
+  const auto tout = tma_place(reg_staging_out(sh, ik, ok, 4, ro ? 1 : M::C, ro ? M::L : 1, 0, M::C, 1), ro);
+  auto at = [&](uint32_t t, uint32_t r) { return (t ^ (r & M::XM)) + (r & ~M::XM); };
+  int excess = 0;
+  std::vector<int> seen(M::TP, 0), out_seen(M::TP, 0);
+  std::vector<int64_t> slot(M::TP, -1);
+  auto tag = [](uint32_t k1, uint32_t v, uint32_t c) { return ((int64_t)k1 * M::NV + v) * M::C + c; };
+  for (uint32_t w = 0; w < 16; ++w) {
+    std::set<uint32_t> read, wrote;
+    for (uint32_t h = 0; h < 2; ++h)
+      for (uint32_t i = 0; i < 4; ++i) {
+        std::vector<uint32_t> la;
+        for (uint32_t l = 0; l < 32; ++l) {
+          const uint32_t x = at(M::load1_t(l, w), M::load1_r(h, i));
+          CHECK(x % 16 == 0 && x + 16 <= bytes, "load %u", x);
+          for (uint32_t u = 0; u < 4; ++u) {
+            const auto a = M::p1(l >> 2, h, u, w);
+            const uint32_t pos = ((l & 3) + 4 * i) * M::NV + a.v;
+            CHECK(a.v < (uint32_t)M::NV && a.c < (uint32_t)M::C, "vector %u %u", a.v, a.c);
+            CHECK(tin[pos * M::C + a.c] == x + 4 * u, "point %u %u staged at %u, read at %u", pos, a.c,
+                  tin[pos * M::C + a.c], x + 4 * u);
+            ++seen[pos * M::C + a.c];
+            read.insert(x + 4 * u);
+          }
+          la.push_back(x);
+        }
+        excess += wavefronts(la, 16) - 4;
+      }
+    // stores: chunk words are the four w, or (h, p) where phase 2 reads operand slots
+    for (uint32_t mt = 0; mt < 2; ++mt)
+      for (uint32_t x = 0; x < 4; ++x) {  // (p, h), or w
+        std::vector<uint32_t> sa;
+        for (uint32_t l = 0; l < 32; ++l) {
+          const uint32_t d = M::WK ? M::store1_r(mt, 0, 0, x) : M::store1_r(mt, x & 1, x >> 1, 0);
+          const uint32_t s = at(M::store1_t(l, w), d);
+          CHECK(s % 16 == 0 && s + 16 <= bytes, "store %u", s);
+          for (uint32_t u = 0; u < 4; ++u) {
+            const uint32_t p = M::WK ? u >> 1 : x & 1, h = M::WK ? u & 1 : x >> 1, ww = M::WK ? x : u;
+            const auto a = M::p1((l & 3) << 1 | p, h, ww, w);
+            const uint32_t k1 = (l >> 2) + 8 * mt;
+            CHECK(slot[s / 4 + u] < 0, "slot written twice");
+            CHECK(M::ex_at(k1, a.v, a.c) == s + 4 * u, "exchange address");
+            slot[s / 4 + u] = tag(k1, a.v, a.c);
+            wrote.insert(s + 4 * u);
+          }
+          sa.push_back(s);
+        }
+        excess += wavefronts(sa, 16) - 4;
+      }
+    CHECK(read == wrote, "phase 1 of warp %u writes other slots than it read", w);
+  }
+  for (int x : seen) CHECK(x == 1, "point loaded %d times", x);
+  for (uint32_t w = 0; w < 16; ++w) {
+    std::set<uint32_t> read, wrote;
+    for (uint32_t j = 0; j < 8; ++j) {
+      std::vector<uint32_t> la;
+      for (uint32_t l = 0; l < 32; ++l) {
+        const uint32_t x = at(M::load2_t(l, w), M::load2_r(j));
+        CHECK(x % 16 == 0 && x + 16 <= bytes, "load %u", x);
+        for (uint32_t u = 0; u < 4 && x + 16 <= bytes; ++u) {
+          const uint32_t unit = M::WK ? j : (j >> 2) * 4 + u, i = M::WK ? u : j & 3;
+          const auto a = M::p2(l >> 2, unit, w);
+          CHECK(a.k1 < 16 && a.n3 < (uint32_t)M::R && a.c < (uint32_t)M::C, "phase 2 vector");
+          const int64_t want = tag(a.k1, M::v_of((l & 3) + 4 * i, a.n3), a.c);
+          CHECK(slot[x / 4 + u] == want, "phase 2 reads %lld for %lld", (long long)slot[x / 4 + u], (long long)want);
+          read.insert(x + 4 * u);
+        }
+        la.push_back(x);
+      }
+      excess += wavefronts(la, 16) - 4;
+    }
+    // outputs, chunk by chunk as run() stores them
+    auto put = [&](uint32_t d, auto who) {  // who(word) -> (mt, p, unit, k3)
+      std::vector<uint32_t> sa;
+      for (uint32_t l = 0; l < 32; ++l) {
+        const uint32_t s = at(M::store2_t(l, w), d);
+        CHECK(s % 16 == 0 && s + 16 <= bytes, "store %u", s);
+        for (uint32_t u = 0; u < 4 && s + 16 <= bytes; ++u) {
+          uint32_t mt, p, unit, k3;
+          who(u, mt, p, unit, k3);
+          const auto a = M::p2((l & 3) << 1 | p, unit, w);
+          const uint32_t pos = a.k1 + 16 * ((l >> 2) + 8 * mt) + 256 * k3;
+          CHECK(tout[pos * M::C + a.c] == s + 4 * u, "output %u %u taken from %u, stored at %u", pos, a.c,
+                tout[pos * M::C + a.c], s + 4 * u);
+          ++out_seen[pos * M::C + a.c];
+          wrote.insert(s + 4 * u);
+        }
+        sa.push_back(s);
+      }
+      excess += wavefronts(sa, 16) - 4;
+    };
+    for (uint32_t mt = 0; mt < 2; ++mt)
+      for (uint32_t x = 0; x < 4; ++x) {
+        if (M::L == 256 && M::KIND == kCC)
+          put(M::store2_r(mt, x & 1, 4 * (x >> 1), 0), [&](uint32_t u, uint32_t& m, uint32_t& p, uint32_t& un, uint32_t& k3) {
+            m = mt, p = x & 1, un = u + 4 * (x >> 1), k3 = 0;
+          });
+        else if (M::L == 256)
+          put(M::store2_r(mt, 0, 2 * x, 0), [&](uint32_t u, uint32_t& m, uint32_t& p, uint32_t& un, uint32_t& k3) {
+            m = mt, p = u & 1, un = 2 * x + (u >> 1), k3 = 0;
+          });
+        else if (M::L == 512)
+          put(M::store2_r(mt, x & 1, 0, x >> 1), [&](uint32_t u, uint32_t& m, uint32_t& p, uint32_t& un, uint32_t& k3) {
+            m = mt, p = x & 1, un = M::KIND == kCC ? u : 2 * u, k3 = x >> 1;
+          });
+        else
+          put(M::store2_r(mt, 0, 0, x), [&](uint32_t u, uint32_t& m, uint32_t& p, uint32_t& un, uint32_t& k3) {
+            m = mt, p = M::KIND == kCC ? 0 : u & 1, un = M::KIND == kCC ? u : 4 * (u >> 1), k3 = x;
+          });
+      }
+    if (M::KIND == kRR) CHECK(read == wrote, "phase 2 of warp %u writes other slots than it read", w);
+  }
+  for (int x : out_seen) CHECK(x == 1, "output written %d times", x);
+  CHECK(excess == 0, "%d wavefronts of bank conflicts", excess);
+  // twiddle tables: every entry set, unit modulus (phase 1)
+  std::vector<float> tab(M::TWB / 4, 7.f);
+  M::fill_twiddles(tab.data());
+  for (size_t i = 0; i < tab.size(); i += 4)
+    for (int p = 0; p < 2; ++p) {
+      const double r = (double)tab[i + p] * tab[i + p] + (double)tab[i + 2 + p] * tab[i + 2 + p];
+      const double want = i * 4 < (size_t)M::TW1B ? 1.0 : 1.0 / M::R / M::R;
+      CHECK(r > want * 0.999 && r < want * 1.001, "twiddle entry %zu", i / 4);
+    }
+  printf("%s tensor cores %s (excess wavefronts %d)\n", g_bad == bad0 ? "ok" : "FAULT", name, excess);
+}
+
+#define W(L, K, PT) check_mma<MmaPass<L, K, PT, false>>(#L " " #K)
 #define V(L, R1, R2, TP, I, O, K, PT) check<RegPass<L, R1, R2, TP, I, O, K, PT, false>>(#L " " #R1 "x" #R2 " " #TP " " #I " " #O " " #K)
 #define ROWS(TP, I, O, K)                                                              \
   V(64, 8, 8, TP, I, O, K, false), V(128, 8, 16, TP, I, O, K, false), V(256, 16, 16, TP, I, O, K, false), \
       V(512, 16, 32, TP, I, O, K, false), V(1024, 32, 32, TP, I, O, K, false)
 
 int main() {
+  W(256, kRR, false), W(512, kRR, false), W(1024, kRR, false);
+  W(256, kRC, false), W(512, kRC, false), W(1024, kRC, false);
+  W(256, kCC, true), W(512, kCC, true), W(1024, kCC, true);
   ROWS(16384, true, true, kRR);
   ROWS(16384, true, true, kRC);
   V(64, 8, 8, 16384, true, true, kCC, false);
