@@ -126,6 +126,8 @@ class Plan:
     Plan(descs=[(shape, batch, in_offset, out_offset), ...])   uneven batch
     """
 
+    _exec_const = None  # see _exec_setup
+
     def __init__(self, shape=None, batch: int = 1, precision: int = PREC_FP16,
                  flags: int = FLAG_NONE, descs=None):
         self._h = ctypes.c_void_p()
@@ -164,8 +166,7 @@ class Plan:
         return inf
 
     def exec_ptr(self, in_ptr: int, out_ptr: int, direction: int = FORWARD, stream: int = 0):
-        _check(lib().mcfftExec(self._h, ctypes.c_void_p(in_ptr), ctypes.c_void_p(out_ptr),
-                               direction, ctypes.c_void_p(stream)), "mcfftExec")
+        _check(lib().mcfftExec(self._h, in_ptr, out_ptr, direction, stream), "mcfftExec")
 
     def exec_host_ptr(self, in_ptr: int, out_ptr: int, direction: int = FORWARD, stream: int = 0):
         """Host buffers in and out (page-locked for overlapped copies): copy
@@ -181,35 +182,56 @@ class Plan:
         Both tensors must be contiguous, on the plan's device, and hold at
         least the plan's input / output bytes (the kernels read and write the
         extents the plan describes)."""
+        if self._exec_const is None or not self._h:
+            self._exec_setup()
+        in_dt, out_dt, in_bytes, out_bytes, elements, dev, index = self._exec_const
+        if dev is None and x.is_cuda:
+            dev, index = self._current_device()
+        if not (x.is_cuda and x.is_contiguous() and x.dtype is in_dt and x.device == dev
+                and x.numel() * x.element_size() >= in_bytes):
+            self._refuse(x, in_dt, dev, in_bytes, "x")
+        if out is None:
+            import torch
+            out = torch.empty(elements, dtype=out_dt, device=dev)
+        if not (out.is_cuda and out.is_contiguous() and out.dtype is out_dt and out.device == dev
+                and out.numel() * out.element_size() >= out_bytes):
+            self._refuse(out, out_dt, dev, out_bytes, "out")
+        rc = self._exec_fn(self._h, x.data_ptr(), out.data_ptr(), direction, self._stream_of(index))
+        if rc != SUCCESS:
+            raise McfftError(rc, "mcfftExec")
+        return out
+
+    def _exec_setup(self):
+        """What exec() checks and passes on each call, fixed by the plan: types,
+        bytes, device.  (Raises if the plan is closed.)"""
         import torch
         inf = self.info()
         split = self.precision == PREC_SPLIT
         in_dt = torch.complex64 if split and not (self.flags & FLAG_INPUT_F16) else torch.complex32
         out_dt = torch.complex64 if split else torch.complex32
-        dev = None
+        dev = None if self.device_index is None else torch.device("cuda", self.device_index)
+        raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+        self._stream_of = raw or (lambda i: torch.cuda.current_stream(i).cuda_stream)
+        self._exec_fn = lib().mcfftExec
+        self._exec_const = (in_dt, out_dt, inf.in_bytes, inf.out_bytes, inf.elements, dev,
+                            self.device_index)
 
-        def need(t, dtype, nbytes, what):
-            nonlocal dev
-            if not (t.is_cuda and t.is_contiguous()):
-                raise ValueError(f"{what} must be a contiguous CUDA tensor")
-            if dev is None:
-                dev = torch.device("cuda", self.device_index if self.device_index is not None
-                                   else torch.cuda.current_device())
-            if t.dtype != dtype:
-                raise ValueError(f"{what} is {t.dtype}; this plan needs {dtype}")
-            if t.device != dev:
-                raise ValueError(f"{what} is on {t.device}; the plan was made on {dev}")
-            have = t.numel() * t.element_size()
-            if have < nbytes:
-                raise ValueError(f"{what} holds {have} bytes; the plan needs {nbytes}")
+    @staticmethod
+    def _current_device():
+        import torch
+        index = torch.cuda.current_device()
+        return torch.device("cuda", index), index
 
-        need(x, in_dt, inf.in_bytes, "x")
-        if out is None:
-            out = torch.empty(inf.elements, dtype=out_dt, device=dev)
-        need(out, out_dt, inf.out_bytes, "out")
-        stream = torch.cuda.current_stream(dev).cuda_stream
-        self.exec_ptr(x.data_ptr(), out.data_ptr(), direction, stream)
-        return out
+    @staticmethod
+    def _refuse(t, dtype, dev, nbytes, what):
+        if not (t.is_cuda and t.is_contiguous()):
+            raise ValueError(f"{what} must be a contiguous CUDA tensor")
+        if t.dtype != dtype:
+            raise ValueError(f"{what} is {t.dtype}; this plan needs {dtype}")
+        if t.device != dev:
+            raise ValueError(f"{what} is on {t.device}; the plan was made on {dev}")
+        have = t.numel() * t.element_size()
+        raise ValueError(f"{what} holds {have} bytes; the plan needs {nbytes}")
 
     def check_status(self):
         _check(lib().mcfftPlanCheckStatus(self._h), "mcfftPlanCheckStatus")
