@@ -53,13 +53,38 @@ __device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], 
   }
 }
 
-template <int L_, int KIND_, bool POST_, bool INV_>
+// The A fragments (the same for every pass of a direction): output half mt,
+// operand half s.
+struct MmaFrags {
+  uint32_t a[2][2][4];
+  template <class A>
+  __device__ __forceinline__ MmaFrags(const A& args, int t) {
+    const uint4* f = args.bmat + (t & 31) * 4;
+#pragma unroll
+    for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        const uint4 x = __ldg(f + mt * 2 + s);
+        a[mt][s][0] = x.x;
+        a[mt][s][1] = x.y;
+        a[mt][s][2] = x.z;
+        a[mt][s][3] = x.w;
+      }
+  }
+};
+
+// TP: 16384 points per tile; 4096 (rows in and out, where a warp needs no
+// other) for small batches.
+template <int L_, int KIND_, bool POST_, bool INV_, int TP_ = 16384>
 struct MmaPass {
-  static constexpr int L = L_, KIND = KIND_, TP = 16384, R = L / 256, NV = L / 16, C = TP / L;
+  static constexpr int L = L_, KIND = KIND_, TP = TP_, R = L / 256, NV = L / 16, C = TP / L;
   static constexpr bool POST = POST_, INV = INV_;
   static_assert(L == 256 || L == 512 || L == 1024, "16 x 16 x R");
   static_assert(!POST || KIND == kCC, "four-step twiddle on column passes");
-  static constexpr int T = 512, NW = 16, NG = 1, NBUF = 3, NFULL = NBUF, THREADS = T + 128;
+  static_assert(TP == 16384 || (TP == 4096 && KIND == kRR), "tile size");
+  static constexpr int T = TP / 32, NW = T / 32, NG = 1;
+  static constexpr bool BIG = T == 512;
+  static constexpr int NBUF = BIG ? 3 : 2, NFULL = NBUF, THREADS = T + (BIG ? 128 : 32), MINB = BIG ? 1 : 3;
   static constexpr int BUF = TP * 4;
   static constexpr bool ROWIN = KIND != kCC;
   // Phase 2 of row-input passes of 256 and 512 points reads the four operand
@@ -236,24 +261,8 @@ struct MmaPass {
   static constexpr int SMEM_BYTES = OFF_BAR + 128 + 1024;
   static_assert(SMEM_BYTES <= 232448, "shared memory budget");
 
-  // The A fragments: output half mt, operand half s.
-  struct State {
-    uint32_t a[2][2][4];
-    template <class A>
-    __device__ __forceinline__ State(const A& args, int t) {
-      const uint4* f = args.bmat + (t & 31) * 4;
-#pragma unroll
-      for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-        for (int s = 0; s < 2; ++s) {
-          const uint4 x = __ldg(f + mt * 2 + s);
-          a[mt][s][0] = x.x;
-          a[mt][s][1] = x.y;
-          a[mt][s][2] = x.z;
-          a[mt][s][3] = x.w;
-        }
-    }
-  };
+  using State = MmaFrags;
+
   // DFT-16 of the unit whose operand slots are b0 .. b3: pairs re[mt], im[mt].
   static __device__ __forceinline__ void unit(const State& st, u32 b0, u32 b1, u32 b2, u32 b3, P2 (&re)[2],
                                               P2 (&im)[2]) {

@@ -1,6 +1,6 @@
 // fft_reg.cuh -- TMA-fed FFT pass kernel whose butterflies stay in registers.
 //
-// One persistent CTA per SM; a tile holds C columns x L points, L = R1 R2,
+// Persistent, one CTA per SM (small tiles: three); a tile holds C columns x L points, L = R1 R2,
 // both radices at most 32.  A thread holds 32 points of the tile in FP32: one
 // 32-point vector, two of 16 or four of 8 (fft_codelets.cuh), so a pass of up
 // to 1024 points is two phases with one exchange through shared memory:
@@ -116,6 +116,7 @@ struct RegPass {
   static constexpr bool PK = OUT16;
   static constexpr int lgC = ilog2c(C), lgNV = ilog2c(NV), lgR1 = ilog2c(R1);
   static constexpr int nc = 10 - ilog2c(L);  // column bits inside a warp (row passes)
+  static_assert(T >= 128 && (T >= 256 || KIND == kRR), "small tiles: rows in and out");
   static_assert(C >= 8, "row swizzle and in-warp columns need eight columns");
   // Column staging: bytes of one point row, and the point rows that share a
   // 128-byte line (1 << h of them).
@@ -128,14 +129,15 @@ struct RegPass {
   // factor doubled for two columns, 16 bytes; FP32 form 8 bytes.
   static constexpr int TWN = PK ? (R1 == 32 ? L / 2 : L) : L;  // entries, k-major, v fastest
   static constexpr int TWB = TWN * (PK ? 16 : 8);
-  static constexpr int NG = 512 / T > 2 ? 2 : 512 / T;  // tiles in work at a time
-  static constexpr int NBUF = BUF <= 32768 ? 5 : 3;
+  static constexpr int NG = T >= 256 ? 512 / T : 1;  // tiles in work at a time
+  static constexpr int NBUF = T >= 256 ? 3 : 2;
   // Load barriers: a ring long enough that one group alone waits on each
   // (tile i and tile i + NFULL go to the same group).  A group may run ahead
   // of the other's tile in the same buffer, and a parity wait is only right
   // for a waiter that has seen the phase before.
   static constexpr int NFULL = NG == 1 ? NBUF : NG * NBUF;
-  static constexpr int THREADS = NG * T + 128;
+  static constexpr bool BIG = NG * T == 512;  // one CTA per SM; else small tiles, several
+  static constexpr int THREADS = NG * T + (BIG ? 128 : 32), MINB = BIG ? 1 : 3;
   static constexpr int OFF_TW = NBUF * BUF;
   static constexpr int OFF_BAR = OFF_TW + TWB;
   static constexpr int SMEM_BYTES = OFF_BAR + 128 + 1024;
@@ -558,7 +560,7 @@ struct RegPass {
 };
 
 template <class P>
-__global__ void __launch_bounds__(P::THREADS, 1) fft_reg(const __grid_constant__ TileArgs a) {
+__global__ void __launch_bounds__(P::THREADS, P::MINB) fft_reg(const __grid_constant__ TileArgs a) {
   constexpr int NG = P::NG, T = P::T, NW = P::NW, NBUF = P::NBUF;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_u = sm100::smem_u32(smem_raw);
@@ -570,40 +572,44 @@ __global__ void __launch_bounds__(P::THREADS, 1) fft_reg(const __grid_constant__
   volatile int* abort_flag = reinterpret_cast<volatile int*>(done + NBUF);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const bool producer = warp == NG * NW;
+  // 32-bit tile arithmetic (the plan refuses more tiles than that)
+  const uint32_t step = gridDim.x, ntiles = (uint32_t)a.ntiles, ncb = (uint32_t)a.col_blocks;
+  const uint32_t mine = ntiles > blockIdx.x ? (ntiles - 1 - blockIdx.x) / step + 1 : 0;
+  auto load = [&](uint32_t i) {
+    const uint32_t t = blockIdx.x + i * step, b = i % NBUF;
+    int32_t crd[5];
+    tile::tile_coords(a.in_cmul, a.in_omul, t % ncb, t / ncb, crd);
+    sm100::mbar_arrive_expect_tx(&full[i % NFULL], a.in_tile_bytes);
+    tile::tma_load(&a.tmap_in, a.in_ndims, crd, base_u + b * P::BUF, &full[i % NFULL]);
+  };
+  // The first loads are issued before the tables are in place.  Under a
+  // programmatic dependent launch the buffers the passes share are touched
+  // only after the wait; the tables are this launch's own constants.
+  uint32_t loaded = 0;
   if (producer) {
     if (lane == 0) {
+      tile::prefetch_tmap(&a.tmap_in);
+      tile::prefetch_tmap(&a.tmap_out);
       for (int f = 0; f < NFULL; ++f) sm100::mbar_init(&full[f], 1);
       for (int b = 0; b < NBUF; ++b) sm100::mbar_init(&done[b], NW);
       *abort_flag = 0;
       sm100::fence_mbar_init();
-      tile::prefetch_tmap(&a.tmap_in);
-      tile::prefetch_tmap(&a.tmap_out);
+      sm100::grid_dep_wait();
+      for (; loaded < mine && loaded < NBUF; ++loaded) load(loaded);
     }
+    __syncwarp();
   } else if (warp < NG * NW) {
     for (int i = tid; i < P::TWB / 16; i += NG * T)
       *reinterpret_cast<float4*>(smem + P::OFF_TW + 16 * i) = __ldg(a.tw + i);
     P::setup(a, smem + P::OFF_TW, tid);
   }
   __syncthreads();
-  // Up to here only this launch's constant tables were read; the buffers the
-  // passes share are touched from here on (programmatic dependent launch).
   sm100::grid_dep_wait();
   sm100::grid_dep_launch();
-  // 32-bit tile arithmetic (the plan refuses more tiles than that)
-  const uint32_t step = gridDim.x, ntiles = (uint32_t)a.ntiles, ncb = (uint32_t)a.col_blocks;
-  const uint32_t mine = ntiles > blockIdx.x ? (ntiles - 1 - blockIdx.x) / step + 1 : 0;
   if (warp >= NG * NW) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 24;");
+    if constexpr (P::BIG) asm volatile("setmaxnreg.dec.sync.aligned.u32 24;");
     if (producer && lane == 0) {
-      auto load = [&](uint32_t i) {
-        const uint32_t t = blockIdx.x + i * step, b = i % NBUF;
-        int32_t crd[5];
-        tile::tile_coords(a.in_cmul, a.in_omul, t % ncb, t / ncb, crd);
-        sm100::mbar_arrive_expect_tx(&full[i % NFULL], a.in_tile_bytes);
-        tile::tma_load(&a.tmap_in, a.in_ndims, crd, base_u + b * P::BUF, &full[i % NFULL]);
-      };
-      uint32_t loaded = 0, i = 0;
-      for (; loaded < mine && loaded < NBUF; ++loaded) load(loaded);
+      uint32_t i = 0;
       for (; i < mine; ++i) {
         const uint32_t b = i % NBUF;
         wait_or_abort(&done[b], (i / NBUF) & 1u, abort_flag);
@@ -623,8 +629,11 @@ __global__ void __launch_bounds__(P::THREADS, 1) fft_reg(const __grid_constant__
       for (; i < loaded; ++i) sm100::mbar_wait_bounded(&full[i % NFULL], (i / NFULL) & 1u, kWaitLimit);
     }
     __syncwarp();
-  } else {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
+    __syncthreads();
+    return;  // the rest belongs to the warps that hold registers for it
+  }
+  {
+    if constexpr (P::BIG) asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
     const int grp = NG == 1 ? 0 : tid / T, t = tid - grp * T;
     const Sync<T> sync{1 + grp};
     const typename P::State st(a, t);

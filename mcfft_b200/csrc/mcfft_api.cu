@@ -376,6 +376,17 @@ bool gather_rows(const layout::Staging& tile_st, int64_t L, int64_t C,
   return true;
 }
 
+// Row passes of few points take 4096-point tiles (four warps, three CTAs per
+// SM), which spread over the SMs and have a quarter of the latency.  Measured
+// on a B200, back-to-back execs, 4096-point against full tiles: 1024 x 8 6.2
+// against 8.2 us, 256 x 1000 4.1 / 7.5, 64 x 5000 4.1 / 8.2, 512 x 5000 8.2 /
+// 10.3, 512 x 9001 14.3 / 14.3.  Past about four full tiles per SM the two
+// tie, and as the first pass of a 2D transform the full tiles are faster
+// (1024^2 x 16: 57.4 against 59.4 us).
+bool small_tiles(const mcfftPlan p, const PassSpec& s) {
+  return s.in_sp == 1 && s.out_sp == 1 && s.L * s.ncols * s.nouter <= int64_t(4) * p->sms * 16384;
+}
+
 // Builds a pass on the TMA-fed kernel.  Returns MCFFT_UNSUPPORTED_SIZE when
 // the shape is outside what that kernel handles (the caller falls back).
 mcfftResult add_tile_pass(mcfftPlan p, const PassSpec& s, int only_tile_points = 0) {
@@ -407,10 +418,11 @@ mcfftResult add_tile_pass(mcfftPlan p, const PassSpec& s, int only_tile_points =
   // 1.33x .. 1.39x on four-step, 2D and 3D transforms, plain 1.04x .. 1.13x).
   // Passes of the batch queue, longer columns and the plain form's 8K-point
   // tiles (small batches) take the tcgen05 tiles.
-  for (int oi = 0; oi < 2 && !k; ++oi) {
+  const int small = small_tiles(p, s) && !only_tile_points ? 4096 : 0;
+  for (int oi = small ? -1 : 0; oi < 2 && !k; ++oi) {
     if (p->queue_planned || indexed) break;
-    const TileKernel* cand =
-        find_reg_kernel((int)s.L, ik, ok, s.posttw, p->split, order[oi], s.in_f16 != 0);
+    const TileKernel* cand = find_reg_kernel((int)s.L, ik, ok, s.posttw, p->split,
+                                             oi < 0 ? small : order[oi], s.in_f16 != 0);
     if (!cand || (s.ncols + cand->C - 1) / cand->C * s.nouter >= (int64_t(1) << 31)) continue;
     layout::Staging si, so;
     reg_stagings(*cand, ik, ok, in_elem, out_elem, s.in_sp, s.in_sc, s.in_so, s.out_sp, s.out_sc,
@@ -481,10 +493,10 @@ mcfftResult add_tile_pass(mcfftPlan p, const PassSpec& s, int only_tile_points =
       float4* tw = nullptr;
       r = plan_alloc(p, &tw, (size_t)k->tw_bytes + (k->mma ? 2048 : 0));
       if (r) return r;
-      if (k->mma) {  // twiddle table, then the matrix fragments
-        std::vector<uint32_t> tab((size_t)k->tw_bytes / 4 + 512);
+      if (k->fill_tw[dir]) {  // twiddle table, then the matrix fragments
+        std::vector<uint32_t> tab((size_t)k->tw_bytes / 4 + (k->mma ? 512 : 0));
         k->fill_tw[dir](reinterpret_cast<float*>(tab.data()));
-        k->fill_frag[dir](tab.data() + k->tw_bytes / 4);
+        if (k->mma) k->fill_frag[dir](tab.data() + k->tw_bytes / 4);
         const cudaError_t e = cudaMemcpy(tw, tab.data(), tab.size() * 4, cudaMemcpyHostToDevice);
         if (e != cudaSuccess) return cuda_fail(e);
         tp.tw[dir] = tw;
@@ -659,6 +671,7 @@ mcfftResult autotune_group(mcfftPlan p, size_t first, int64_t points) {
     // indexed passes keep the default shape (they run only in the batch
     // queue, which the tuner's single-pass timing does not model)
     if (!p->passes[i].tiled || p->passes[i].in_tab || p->passes[i].out_tab) continue;
+    if (p->passes[i].tp.k->tile_points == 4096) continue;  // chosen by size (small_tiles)
     const int rec = wisdom_find(gk + "\t" + pass_key(p->passes[i].spec));
     if (!rec) {
       todo.push_back(i);

@@ -43,10 +43,10 @@ TileKernel make_reg() {
   return k;
 }
 
-template <int L, int KIND, bool POST>
+template <int L, int KIND, bool POST, int TP = 16384>
 TileKernel make_mma() {
-  using P = reg::MmaPass<L, KIND, POST, false>;
-  using Q = reg::MmaPass<L, KIND, POST, true>;
+  using P = reg::MmaPass<L, KIND, POST, false, TP>;
+  using Q = reg::MmaPass<L, KIND, POST, true, TP>;
   TileKernel k{reinterpret_cast<const void*>(&reg::fft_reg<P>), L, P::R, P::C, POST, false, P::THREADS,
                P::SMEM_BYTES, 0, P::TP, true};
   k.fn_inv = reinterpret_cast<const void*>(&reg::fft_reg<Q>);

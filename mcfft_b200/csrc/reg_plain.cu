@@ -1,4 +1,5 @@
-// reg_plain.cu -- plain-form (FP16) register pass kernels, 16K-point tiles:
+// reg_plain.cu -- plain-form (FP16) register pass kernels, 16K-point tiles
+// (4096 points for small batches of rows):
 // 64 and 128 points as two register phases (RegPass), 256 to 1024 with the
 // radix-16 stages on the tensor cores (MmaPass).
 #include "reg_pass.h"
@@ -26,7 +27,12 @@ const std::vector<TileKernel>& reg_registry_plain() {
       make_mma<1024, reg::kCC, false>(),
       make_mma<256, reg::kCC, true>(),
       make_mma<512, reg::kCC, true>(),
-      make_mma<1024, reg::kCC, true>()};
+      make_mma<1024, reg::kCC, true>(),
+      make_reg<64, 8, 8, 4096, true, true, reg::kRR, false>(),
+      make_reg<128, 8, 16, 4096, true, true, reg::kRR, false>(),
+      make_mma<256, reg::kRR, false, 4096>(),
+      make_mma<512, reg::kRR, false, 4096>(),
+      make_mma<1024, reg::kRR, false, 4096>()};
   return v;
 }
 

@@ -15,7 +15,12 @@ const std::vector<TileKernel>& reg_registry_split16() {
       make_reg<128, 8, 16, 8192, true, false, reg::kCC, true>(),
       make_reg<256, 16, 16, 8192, true, false, reg::kCC, true>(),
       make_reg<512, 32, 16, 8192, true, false, reg::kCC, true>(),
-      make_reg<1024, 32, 32, 8192, true, false, reg::kCC, true>()};
+      make_reg<1024, 32, 32, 8192, true, false, reg::kCC, true>(),
+      // small batches of rows
+      make_reg<64, 8, 8, 4096, true, false, reg::kRR, false>(),
+      make_reg<128, 8, 16, 4096, true, false, reg::kRR, false>(),
+      make_reg<256, 16, 16, 4096, true, false, reg::kRR, false>(),
+      make_reg<512, 16, 32, 4096, true, false, reg::kRR, false>()};
   return v;
 }
 

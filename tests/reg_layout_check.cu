@@ -183,7 +183,7 @@ void check_mma(const char* name) {
   std::vector<int> seen(M::TP, 0), out_seen(M::TP, 0);
   std::vector<int64_t> slot(M::TP, -1);
   auto tag = [](uint32_t k1, uint32_t v, uint32_t c) { return ((int64_t)k1 * M::NV + v) * M::C + c; };
-  for (uint32_t w = 0; w < 16; ++w) {
+  for (uint32_t w = 0; w < (uint32_t)M::NW; ++w) {
     std::set<uint32_t> read, wrote;
     for (uint32_t h = 0; h < 2; ++h)
       for (uint32_t i = 0; i < 4; ++i) {
@@ -228,7 +228,7 @@ void check_mma(const char* name) {
     CHECK(read == wrote, "phase 1 of warp %u writes other slots than it read", w);
   }
   for (int x : seen) CHECK(x == 1, "point loaded %d times", x);
-  for (uint32_t w = 0; w < 16; ++w) {
+  for (uint32_t w = 0; w < (uint32_t)M::NW; ++w) {
     std::set<uint32_t> read, wrote;
     for (uint32_t j = 0; j < 8; ++j) {
       std::vector<uint32_t> la;
@@ -303,6 +303,7 @@ void check_mma(const char* name) {
 }
 
 #define W(L, K, PT) check_mma<MmaPass<L, K, PT, false>>(#L " " #K)
+#define WS(L) check_mma<MmaPass<L, kRR, false, false, 4096>>(#L " small")
 #define V(L, R1, R2, TP, I, O, K, PT) check<RegPass<L, R1, R2, TP, I, O, K, PT, false>>(#L " " #R1 "x" #R2 " " #TP " " #I " " #O " " #K)
 #define ROWS(TP, I, O, K)                                                              \
   V(64, 8, 8, TP, I, O, K, false), V(128, 8, 16, TP, I, O, K, false), V(256, 16, 16, TP, I, O, K, false), \
@@ -310,6 +311,7 @@ void check_mma(const char* name) {
 
 int main() {
   W(256, kRR, false), W(512, kRR, false), W(1024, kRR, false);
+  WS(256), WS(512), WS(1024);
   W(256, kRC, false), W(512, kRC, false), W(1024, kRC, false);
   W(256, kCC, true), W(512, kCC, true), W(1024, kCC, true);
   ROWS(16384, true, true, kRR);
@@ -322,6 +324,9 @@ int main() {
   ROWS(8192, false, false, kRR);
   ROWS(8192, false, false, kRC);
   ROWS(8192, true, false, kRR);
+  V(64, 8, 8, 4096, true, true, kRR, false), V(128, 8, 16, 4096, true, true, kRR, false);
+  V(64, 8, 8, 4096, false, false, kRR, false), V(128, 8, 16, 4096, false, false, kRR, false);
+  V(256, 16, 16, 4096, false, false, kRR, false), V(512, 16, 32, 4096, false, false, kRR, false);
   V(64, 8, 8, 8192, false, false, kCC, false);
   V(128, 8, 16, 8192, false, false, kCC, false);
   V(256, 16, 16, 8192, false, false, kCC, false);

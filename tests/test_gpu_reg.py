@@ -60,7 +60,16 @@ def _check(shape, batch, form, direction):
 @pytest.mark.parametrize("form", list(FORMS))
 @pytest.mark.parametrize("n", [64, 128, 256, 512, 1024])
 def test_rows(n, form, direction):
-    _check((n,), (9 << 20) // n + 3, form, direction)
+    _check((n,), (10 << 20) // n + 3, form, direction)
+
+
+@pytest.mark.parametrize("direction", [mc.FORWARD, mc.INVERSE])
+@pytest.mark.parametrize("form", list(FORMS))
+@pytest.mark.parametrize("n,batch", [(64, 1), (64, 40001), (128, 70), (256, 17), (256, 12345), (512, 9001),
+                                     (1024, 3), (1024, 2000)])
+def test_few_rows(n, batch, form, direction):
+    """4096-point tiles: from one transform up to several tiles per CTA."""
+    _check((n,), batch, form, direction)
 
 
 @pytest.mark.parametrize("direction", [mc.FORWARD, mc.INVERSE])
