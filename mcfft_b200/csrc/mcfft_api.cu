@@ -384,6 +384,7 @@ bool gather_rows(const layout::Staging& tile_st, int64_t L, int64_t C,
 // tie, and as the first pass of a 2D transform the full tiles are faster
 // (1024^2 x 16: 57.4 against 59.4 us).
 bool small_tiles(const mcfftPlan p, const PassSpec& s) {
+  if (s.L == 4096) return true;  // the register kernel of this length has one tile size
   return s.in_sp == 1 && s.out_sp == 1 && s.L * s.ncols * s.nouter <= int64_t(4) * p->sms * 16384;
 }
 

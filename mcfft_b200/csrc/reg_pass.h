@@ -3,6 +3,7 @@
 #pragma once
 #include "fft_mma.cuh"
 #include "fft_reg.cuh"
+#include "fft_reg4096.cuh"
 #include "tile_pass.h"
 
 namespace mcfft {
@@ -57,6 +58,36 @@ TileKernel make_mma() {
   k.fill_tw[1] = &Q::fill_twiddles;
   k.fill_frag[0] = &P::fill_fragments;
   k.fill_frag[1] = &Q::fill_fragments;
+  return k;
+}
+
+// 4096-point rows (fft_reg4096.cuh).
+inline TileKernel make_mma4096() {
+  using P = reg::Mma4096<false>;
+  using Q = reg::Mma4096<true>;
+  TileKernel k{reinterpret_cast<const void*>(&reg::fft_reg<P>), 4096, 16, 1, false, false, P::THREADS,
+               P::SMEM_BYTES, 0, P::TP, true};
+  k.fn_inv = reinterpret_cast<const void*>(&reg::fft_reg<Q>);
+  k.reg_kind = reg::kRR;
+  k.tw_bytes = P::TWB;
+  k.mma = true;
+  k.fill_tw[0] = &P::fill_twiddles;
+  k.fill_tw[1] = &Q::fill_twiddles;
+  k.fill_frag[0] = &P::fill_fragments;
+  k.fill_frag[1] = &Q::fill_fragments;
+  return k;
+}
+template <bool IN16>
+TileKernel make_reg4096() {
+  using P = reg::Reg4096<IN16, false>;
+  using Q = reg::Reg4096<IN16, true>;
+  TileKernel k{reinterpret_cast<const void*>(&reg::fft_reg<P>), 4096, 16, 1, false, true, P::THREADS,
+               P::SMEM_BYTES, 0, P::TP, IN16};
+  k.fn_inv = reinterpret_cast<const void*>(&reg::fft_reg<Q>);
+  k.reg_kind = reg::kRR;
+  k.tw_bytes = P::TWB;
+  k.fill_tw[0] = &P::fill_twiddles;
+  k.fill_tw[1] = &Q::fill_twiddles;
   return k;
 }
 

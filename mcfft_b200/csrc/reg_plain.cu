@@ -32,7 +32,8 @@ const std::vector<TileKernel>& reg_registry_plain() {
       make_reg<128, 8, 16, 4096, true, true, reg::kRR, false>(),
       make_mma<256, reg::kRR, false, 4096>(),
       make_mma<512, reg::kRR, false, 4096>(),
-      make_mma<1024, reg::kRR, false, 4096>()};
+      make_mma<1024, reg::kRR, false, 4096>(),
+      make_mma4096()};
   return v;
 }
 

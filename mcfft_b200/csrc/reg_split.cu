@@ -30,7 +30,8 @@ const std::vector<TileKernel>& reg_registry_split() {
       make_reg<64, 8, 8, 4096, false, false, reg::kRR, false>(),
       make_reg<128, 8, 16, 4096, false, false, reg::kRR, false>(),
       make_reg<256, 16, 16, 4096, false, false, reg::kRR, false>(),
-      make_reg<512, 16, 32, 4096, false, false, reg::kRR, false>()};
+      make_reg<512, 16, 32, 4096, false, false, reg::kRR, false>(),
+      make_reg4096<false>()};
   return v;
 }
 

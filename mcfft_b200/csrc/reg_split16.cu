@@ -20,7 +20,8 @@ const std::vector<TileKernel>& reg_registry_split16() {
       make_reg<64, 8, 8, 4096, true, false, reg::kRR, false>(),
       make_reg<128, 8, 16, 4096, true, false, reg::kRR, false>(),
       make_reg<256, 16, 16, 4096, true, false, reg::kRR, false>(),
-      make_reg<512, 16, 32, 4096, true, false, reg::kRR, false>()};
+      make_reg<512, 16, 32, 4096, true, false, reg::kRR, false>(),
+      make_reg4096<true>()};
   return v;
 }
 

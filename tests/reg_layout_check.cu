@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "../mcfft_b200/csrc/fft_mma.cuh"
+#include "../mcfft_b200/csrc/fft_reg4096.cuh"
 #include "../mcfft_b200/csrc/reg_staging.h"
 
 using namespace mcfft;
@@ -302,6 +303,131 @@ void check_mma(const char* name) {
   printf("%s tensor cores %s (excess wavefronts %d)\n", g_bad == bad0 ? "ok" : "FAULT", name, excess);
 }
 
+// 4096-point rows, plain form: the three phases' chunks.
+static void check_mma4096() {
+  using M = Mma4096<false>;
+  const int bad0 = g_bad;
+  const RegShape sh{4096, 16, 1, 0, true};
+  const auto tin = tma_place(reg_staging_in(sh, layout::ROW, 4, 1, 4096, 0, 1, 1), true);
+  const auto tout = tma_place(reg_staging_out(sh, layout::ROW, layout::ROW, 4, 1, 4096, 0, 1, 1), true);
+  auto at = [&](uint32_t t, uint32_t r) { return (t ^ (r & M::XM)) + (r & ~M::XM); };
+  int excess = 0;
+  std::vector<int> slot1(4096, -1), slot2(4096, -1), out(4096, 0), seen(4096, 0);
+  auto chunk = [&](uint32_t w, auto addr, auto word) {  // one access of warp w
+    std::vector<uint32_t> a;
+    for (uint32_t l = 0; l < 32; ++l) {
+      const uint32_t x = addr(l);
+      CHECK(x % 16 == 0 && x + 16 <= 16384, "access %u", x);
+      for (uint32_t u = 0; u < 4 && x + 16 <= 16384; ++u) word(l, u, x / 4 + u);
+      a.push_back(x);
+    }
+    (void)w;
+    excess += wavefronts(a, 16) - 4;
+  };
+  for (uint32_t w = 0; w < 4; ++w) {
+    std::set<uint32_t> rd, wr;
+    for (uint32_t j = 0; j < 8; ++j)
+      chunk(w, [&](uint32_t l) { return at(M::load1_t(l, w), M::load1_r(j >> 2, j & 3)); },
+            [&](uint32_t l, uint32_t u, uint32_t s) {
+              const auto a = M::p1(l >> 2, j >> 2, u, w);
+              const uint32_t pos = ((l & 3) + 4 * (j & 3)) * 256 + a.x * 16 + a.y;
+              CHECK(tin[pos] == 4 * s, "point %u", pos);
+              ++seen[pos];
+              rd.insert(s);
+            });
+    for (uint32_t e = 0; e < 8; ++e)
+      chunk(w, [&](uint32_t l) { return at(M::store1_t(l, w), M::store1_r(e & 1, (e >> 1) & 1, e >> 2)); },
+            [&](uint32_t l, uint32_t u, uint32_t s) {
+              const auto a = M::p1((l & 3) << 1 | ((e >> 1) & 1), e >> 2, u, w);
+              CHECK(slot1[s] < 0, "slot written twice");
+              slot1[s] = (int)(((l >> 2) + 8 * (e & 1)) * 256 + a.x * 16 + a.y);
+              wr.insert(s);
+            });
+    CHECK(rd == wr, "phase 1 leaves its slots");
+  }
+  for (uint32_t w = 0; w < 4; ++w) {
+    std::set<uint32_t> rd, wr;
+    for (uint32_t j = 0; j < 8; ++j)
+      chunk(w, [&](uint32_t l) { return at(M::load2_t(l, w), M::load2_r(j >> 2, j & 3)); },
+            [&](uint32_t l, uint32_t u, uint32_t s) {
+              const auto a = M::p2(l >> 2, j >> 2, u, w);
+              CHECK(slot1[s] == (int)(a.x * 256 + ((l & 3) + 4 * (j & 3)) * 16 + a.y), "phase 2 load");
+              rd.insert(s);
+            });
+    for (uint32_t e = 0; e < 8; ++e)
+      chunk(w, [&](uint32_t l) { return at(M::store2_t(l, w), M::store2_r(e & 1, e >> 1)); },
+            [&](uint32_t l, uint32_t u, uint32_t s) {  // words: h + 2 p is n3's upper half, stored as p + 2 h
+              const auto a = M::p2((l & 3) << 1 | (u & 1), u >> 1, e >> 1, w);
+              CHECK(slot2[s] < 0, "slot written twice");
+              slot2[s] = (int)(a.x * 256 + ((l >> 2) + 8 * (e & 1)) * 16 + a.y);
+              wr.insert(s);
+            });
+    CHECK(rd == wr, "phase 2 leaves its slots");
+  }
+  for (uint32_t w = 0; w < 4; ++w) {
+    for (uint32_t j = 0; j < 8; ++j)
+      chunk(w, [&](uint32_t l) { return at(M::load3_t(l, w), M::load3_r(j)); },
+            [&](uint32_t l, uint32_t u, uint32_t s) {
+              const auto a = M::p3(l >> 2, j, w);
+              CHECK(slot2[s] == (int)(a.x * 256 + a.y * 16 + (l & 3) + 4 * u), "phase 3 load");
+            });
+    for (uint32_t e = 0; e < 8; ++e)
+      chunk(w, [&](uint32_t l) { return at(M::store3_t(l, w), M::store3_r(e & 1, e >> 1 << 1)); },
+            [&](uint32_t l, uint32_t u, uint32_t s) {
+              const auto a = M::p3((l & 3) << 1 | (u & 1), (e >> 1 << 1) | u >> 1, w);
+              const uint32_t pos = a.x + 16 * a.y + 256 * ((l >> 2) + 8 * (e & 1));
+              CHECK(tout[pos] == 4 * s, "output %u", pos);
+              ++out[pos];
+            });
+  }
+  for (int i = 0; i < 4096; ++i) CHECK(seen[i] == 1 && out[i] == 1, "point %d: %d loads, %d stores", i, seen[i], out[i]);
+  CHECK(excess == 0, "%d wavefronts of bank conflicts", excess);
+  printf("%s 4096-point rows, plain\n", g_bad == bad0 ? "ok" : "FAULT");
+}
+
+// 4096-point rows, FP32 exchange.
+static void check_reg4096() {
+  using M = Reg4096<false, false>;
+  const int bad0 = g_bad;
+  const RegShape sh{4096, 16, 1, 0, false};
+  const auto tin = tma_place(reg_staging_in(sh, layout::ROW, 8, 1, 4096, 0, 1, 1), true);
+  for (uint32_t p = 0; p < 4096; ++p) CHECK(tin[p] == 8 * p, "natural order");
+  int excess = 0;
+  std::vector<int> n1(4096, 0), out(4096, 0), slot(4096, -1);
+  for (uint32_t w = 0; w < 4; ++w)
+    for (uint32_t j = 0; j < 2; ++j)
+      for (uint32_t k = 0; k < 16; ++k) {
+        std::vector<uint32_t> a, b, c, d;
+        for (uint32_t l = 0; l < 32; ++l) {
+          const uint32_t t = w * 32 + l, x = M::xd(t), y = M::yd(t, j);
+          a.push_back((k * 256 + y * 16 + x) * 8);            // phase 1 in and out, phase 3 out
+          b.push_back((y * 256 + k * 16 + x) * 8);            // phase 2 in
+          c.push_back(M::ex2_at(y, k, x));                    // phase 2 out
+          CHECK(c.back() == M::ex2_at(y, 0, x) + k * 128, "phase 2 store offset");
+          ++n1[a.back() / 8];
+          ++out[a.back() / 8];
+          CHECK(slot[c.back() / 8] < 0 && c.back() / 128 == b.back() / 128, "phase 2 slot");
+          slot[c.back() / 8] = (int)(y * 256 + k * 16 + x);
+        }
+        excess += wavefronts(a, 8) - 2 + wavefronts(b, 8) - 2 + wavefronts(c, 8) - 2;
+      }
+  for (uint32_t w = 0; w < 4; ++w)
+    for (uint32_t j = 0; j < 2; ++j)
+      for (uint32_t n = 0; n < 8; ++n) {
+        std::vector<uint32_t> a;
+        for (uint32_t l = 0; l < 32; ++l) {
+          const uint32_t t = w * 32 + l, k1 = M::xd(t), k2 = M::yd(t, j), x = M::ex2_at(k1, k2, 0) ^ (n << 4);
+          for (uint32_t u = 0; u < 2; ++u)
+            CHECK(slot[x / 8 + u] == (int)(k1 * 256 + k2 * 16 + 2 * n + u), "phase 3 load");
+          a.push_back(x);
+        }
+        excess += wavefronts(a, 16) - 4;
+      }
+  for (int i = 0; i < 4096; ++i) CHECK(n1[i] == 1 && out[i] == 1, "point %d", i);
+  CHECK(excess == 0, "%d wavefronts of bank conflicts", excess);
+  printf("%s 4096-point rows, FP32 exchange\n", g_bad == bad0 ? "ok" : "FAULT");
+}
+
 #define W(L, K, PT) check_mma<MmaPass<L, K, PT, false>>(#L " " #K)
 #define WS(L) check_mma<MmaPass<L, kRR, false, false, 4096>>(#L " small")
 #define V(L, R1, R2, TP, I, O, K, PT) check<RegPass<L, R1, R2, TP, I, O, K, PT, false>>(#L " " #R1 "x" #R2 " " #TP " " #I " " #O " " #K)
@@ -310,6 +436,8 @@ void check_mma(const char* name) {
       V(512, 16, 32, TP, I, O, K, false), V(1024, 32, 32, TP, I, O, K, false)
 
 int main() {
+  check_mma4096();
+  check_reg4096();
   W(256, kRR, false), W(512, kRR, false), W(1024, kRR, false);
   WS(256), WS(512), WS(1024);
   W(256, kRC, false), W(512, kRC, false), W(1024, kRC, false);

@@ -66,7 +66,7 @@ def test_rows(n, form, direction):
 @pytest.mark.parametrize("direction", [mc.FORWARD, mc.INVERSE])
 @pytest.mark.parametrize("form", list(FORMS))
 @pytest.mark.parametrize("n,batch", [(64, 1), (64, 40001), (128, 70), (256, 17), (256, 12345), (512, 9001),
-                                     (1024, 3), (1024, 2000)])
+                                     (1024, 3), (1024, 2000), (4096, 1), (4096, 5), (4096, 1501)])
 def test_few_rows(n, batch, form, direction):
     """4096-point tiles: from one transform up to several tiles per CTA."""
     _check((n,), batch, form, direction)
