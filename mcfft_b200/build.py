@@ -27,7 +27,7 @@ SOURCES = ["tables.cu", "pass_kernels.cu", "tile_pass.cu", "tile_split.cu", "que
            "queue_split.cu", "fused.cu",
            "reg_pass.cu", "reg_plain.cu", "reg_split.cu", "reg_split16.cu", "layout.cpp", "mcfft_api.cu", "noalloc.cu", "norms.cu"]
 HEADERS = ["sm100_ptx.cuh", "tail_layout.h", "fft_pass.cuh", "fft_pass_split.cuh", "fft_tile.cuh",
-           "fft_tile_split.cuh", "fft_codelets.cuh", "fft_reg.cuh", "fft_mma.cuh", "fft_reg4096.cuh", "reg_pass.h",
+           "fft_tile_split.cuh", "fft_codelets.cuh", "fft_reg.cuh", "fft_mma.cuh", "fft_rows.cuh", "reg_pass.h",
            "reg_staging.h", "fft_queue.cuh", "queue.h", "queue_order.h", "host_schedule.h",
            "tile_pass.h", "layout.h", "mcfft_internal.h"]
 

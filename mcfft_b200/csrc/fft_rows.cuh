@@ -1,6 +1,7 @@
-// fft_reg4096.cuh -- 4096-point row passes (a 1D transform of 4096 points in
-// one pass) as three radix-16 phases, one transform per tile and four warps.
+// fft_rows.cuh -- row passes of 4096 and 2048 points (1D transforms of these
+// lengths in one pass), a transform to four (two) warps.
 //
+// 4096 points: three radix-16 phases,
 //   n = 256 n1 + 16 n2 + n3, X[k1 + 16 k2 + 256 k3]
 //   phase 1  DFT-16 over n1, twiddle W_4096^(k1 (16 n2 + n3))
 //   phase 2  DFT-16 over n2, twiddle W_256^(k2 n3)
@@ -11,26 +12,36 @@
 // (FP16 input with FP32 exchange: four), three or four CTAs per SM so that
 // their phases overlap: such batches are small more often than not, and a
 // 16K-point tile of four transforms (fft_tile.cuh) leaves most SMs idle and
-// takes four times as long per tile.
+// takes four times as long per tile.  The one-launch kernel of uneven batches
+// runs four transforms per 16K-point tile.
+//
+// 2048 points (plain form): 16 x 16 x 8, two phases as MmaPass with the
+// radix-8 step in registers, eight transforms per 16K-point tile.  Bound by
+// HBM from a few thousand transforms: 20000 in 70.3 us (4.7 TB/s), 79.5 on the
+// tcgen05 tile of four columns; 3000 in 18.5 against 23.6 us; as the rows of
+// 2048^2 x 4, 65.1 against 73.7 us in all.
 #pragma once
 #include "fft_mma.cuh"
 
 namespace mcfft {
 namespace reg {
 
-template <int T>
-__device__ __forceinline__ void group_bar() {
-  asm volatile("bar.sync 1, %0;" ::"n"(T) : "memory");
+// Barrier of the N threads of one transform (id: one per transform in work).
+template <int N>
+__device__ __forceinline__ void col_bar(int id) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(N) : "memory");
 }
 
 // Plain form: the phases of MmaPass, every shared access 16 bytes wide and
 // free of bank conflicts (tests/reg_layout_check.cu).
-template <bool INV_>
+template <bool INV_, int TP_ = 4096>
 struct Mma4096 {
   using u32 = uint32_t;
-  static constexpr int L = 4096, KIND = kRR, TP = 4096, R = 16, C = 1, EI = 4, EO = 4;
-  static constexpr bool POST = false, INV = INV_, BIG = false;
-  static constexpr int T = 128, NW = 4, NG = 1, NBUF = 2, NFULL = 2, THREADS = T + 32, MINB = 4;
+  static constexpr int L = 4096, KIND = kRR, TP = TP_, R = 16, C = TP / L, EI = 4, EO = 4;
+  static constexpr bool POST = false, INV = INV_, BIG = C == 4;
+  static_assert(C == 1 || C == 4, "tile size");
+  static constexpr int T = TP / 32, NW = T / 32, NG = 1, NBUF = BIG ? 3 : 2, NFULL = NBUF;
+  static constexpr int THREADS = T + (BIG ? 128 : 32), MINB = BIG ? 1 : 4;
   static constexpr int BUF = TP * 4;
   using State = MmaFrags;
   static __host__ __device__ constexpr u32 bit(u32 x, int b) { return (x >> b) & 1u; }
@@ -122,7 +133,7 @@ struct Mma4096 {
   // over vector bit 0) at ((warp * 4 + mt * 2 + h) * 32 + lane), its step
   // W_4096^k1 (doubled) at 512 + k1; phase 2: pairs at 528 + (mt * 8 + h * 4 +
   // w) * 8 + g.  16-byte entries.
-  static constexpr int TWB = (512 + 16 + 128) * 16;
+  static constexpr int TWB = (512 + 16 + 128) * 16, TABB = TWB;
   static constexpr int OFF_TW = NBUF * BUF, OFF_BAR = OFF_TW + TWB;
   static constexpr int SMEM_BYTES = OFF_BAR + 128 + 1024;
   static void fill_twiddles(float* out) {
@@ -162,7 +173,9 @@ struct Mma4096 {
   template <class A>
   static __device__ __forceinline__ void run(const A&, const State& st, u32 sb, u32 tws, int t, u32,
                                              const Sync<T>&) {
-    const u32 lane = t & 31, warp = t >> 5, g = lane >> 2;
+    const u32 lane = t & 31, warp = (t >> 5) & 3u, g = lane >> 2;
+    const int bar = 4 + (t >> 7);
+    sb += (t >> 7) * 16384;
     u32 x[8][4];
     {
       const u32 lb = sb + load1_t(lane, warp), sp = sb + store1_t(lane, warp);
@@ -199,7 +212,7 @@ struct Mma4096 {
           for (int p = 0; p < 2; ++p) M::put(sp, store1_r(mt, p, h), o[mt][p]);
       }
     }
-    group_bar<T>();
+    col_bar<128>(bar);
     {
       const u32 lb = sb + load2_t(lane, warp), sp = sb + store2_t(lane, warp);
 #pragma unroll
@@ -223,12 +236,12 @@ struct Mma4096 {
         for (int mt = 0; mt < 2; ++mt) M::put(sp, store2_r(mt, w), o[mt]);
       }
     }
-    group_bar<T>();
+    col_bar<128>(bar);
     {
       const u32 lb = sb + load3_t(lane, warp), sp = sb + store3_t(lane, warp);
 #pragma unroll
       for (int u = 0; u < 8; ++u) get(lb, load3_r(u), x[u]);
-      group_bar<T>();
+      col_bar<128>(bar);
 #pragma unroll
       for (int uu = 0; uu < 8; uu += 2) {
         u32 o[2][4];
@@ -303,7 +316,7 @@ struct Reg4096 {
           im[j][n] = z.y;
         }
       }
-      if constexpr (EI != EO) group_bar<T>();
+      if constexpr (EI != EO) col_bar<128>(4);
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
         const u32 y = yd(t, j), b = sb + (y * 16 + x) * 8;
@@ -318,7 +331,7 @@ struct Reg4096 {
         }
       }
     }
-    group_bar<T>();
+    col_bar<128>(4);
     {
       float re[2][16], im[2][16];
 #pragma unroll
@@ -346,7 +359,7 @@ struct Reg4096 {
         }
       }
     }
-    group_bar<T>();
+    col_bar<128>(4);
     {
       float re[2][16], im[2][16];
 #pragma unroll
@@ -361,13 +374,188 @@ struct Reg4096 {
           im[j][2 * n + 1] = z.w;
         }
       }
-      group_bar<T>();
+      col_bar<128>(4);
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
         const u32 b = sb + (yd(t, j) * 16 + x) * 8;
         Dft<16, INV, float>::run(re[j], im[j]);
 #pragma unroll
         for (int k = 0; k < 16; ++k) tile::sts64(b + k * 256 * 8, make_float2(re[j][k], im[j][k]));
+      }
+    }
+  }
+};
+
+// 2048 points, plain form.
+template <bool INV_>
+struct Mma2048 {
+  using u32 = uint32_t;
+  static constexpr int L = 2048, KIND = kRR, TP = 16384, R = 8, C = 8, EI = 4, EO = 4;
+  static constexpr bool POST = false, INV = INV_, BIG = true;
+  static constexpr int T = 512, NW = 16, NG = 1, NBUF = 3, NFULL = 3, THREADS = T + 128, MINB = 1;
+  static constexpr int BUF = TP * 4;
+  using State = MmaFrags;
+  static __host__ __device__ constexpr u32 bit(u32 x, int b) { return (x >> b) & 1u; }
+
+  // n = 128 n1 + 8 n2 + n3; 128-byte rows of 32 points, rows 16 (n2 >> 2) + n1
+  // within a transform; the output in natural order.
+  static __host__ __device__ constexpr u32 in_at(u32 n1, u32 n2, u32 n3) {
+    return ((n2 >> 2) * 16 + n1) * 128 + ((((n2 & 3u) << 1 | n3 >> 2) ^ (n1 & 7u)) << 4) + (n3 & 3u) * 4;
+  }
+  static __host__ __device__ constexpr u32 ex_at(u32 k1, u32 n2, u32 n3) {
+    return ((n2 >> 2) * 16 + k1) * 128 + ((((n2 & 3u) << 1 | n3 >> 2) ^ (bit(k1, 0) * 5u)) << 4) + (n3 & 3u) * 4;
+  }
+  static __host__ __device__ constexpr u32 out_at(u32 k1, u32 k2, u32 k3) {
+    const u32 pos = k1 + 16 * k2 + 256 * k3, row = pos >> 5;
+    return row * 128 + ((((pos >> 2) ^ row) & 7u) << 4) + (pos & 3u) * 4;
+  }
+  struct XY {
+    u32 x, y;
+  };
+  // phase 1: (n2, n3); phase 2: (k1, n3)
+  static __host__ __device__ constexpr XY p1(u32 g, u32 h, u32 w, u32 warp) {
+    return {bit(g, 1) | bit(g, 0) << 1 | h << 2 | warp << 3, w | bit(g, 2) << 2};
+  }
+  static __host__ __device__ constexpr XY p2(u32 g, u32 h, u32 w, u32 warp) {
+    return {bit(g, 0) | bit(g, 1) << 1 | warp << 2 | bit(g, 2) << 3, w | h << 2};
+  }
+  static constexpr u32 XM = 0x70u;
+  static __host__ __device__ constexpr u32 load1_t(u32 lane, u32 warp) {
+    const XY a = p1(lane >> 2, 0, 0, warp);
+    return in_at(lane & 3u, a.x, a.y);
+  }
+  static __host__ __device__ constexpr u32 load1_r(u32 h, u32 i) {
+    const XY a = p1(0, h, 0, 0);
+    return in_at(4 * i, a.x, a.y);
+  }
+  static __host__ __device__ constexpr u32 store1_t(u32 lane, u32 warp) {
+    const XY a = p1((lane & 3u) << 1, 0, 0, warp);
+    return ex_at(lane >> 2, a.x, a.y);
+  }
+  static __host__ __device__ constexpr u32 store1_r(u32 mt, u32 p, u32 h) {
+    const XY a = p1(p, h, 0, 0);
+    return ex_at(8 * mt, a.x, a.y);
+  }
+  static __host__ __device__ constexpr u32 load2_t(u32 lane, u32 warp) {
+    const XY a = p2(lane >> 2, 0, 0, warp);
+    return ex_at(a.x, lane & 3u, a.y);
+  }
+  static __host__ __device__ constexpr u32 load2_r(u32 h, u32 i) {
+    const XY a = p2(0, h, 0, 0);
+    return ex_at(a.x, 4 * i, a.y);
+  }
+  static __host__ __device__ constexpr u32 store2_t(u32 lane, u32 warp) {
+    const XY a = p2((lane & 3u) << 1, 0, 0, warp);
+    return out_at(a.x, lane >> 2, 0);
+  }
+  static __host__ __device__ constexpr u32 store2_r(u32 mt, u32 k3) { return out_at(0, 8 * mt, k3); }
+
+  // Phase 1: chain starts (pairs over vector bit 0) at ((warp * 4 + mt * 2 + h)
+  // * 32 + lane), steps W_2048^k1 at 256 + k1; phase 2: W_128^(k2 n3) / 8,
+  // doubled, at 272 + ((n3 - 1) * 2 + mt) * 8 + g.
+  static constexpr int TWB = (256 + 16 + 112) * 16, TABB = TWB;
+  static constexpr int OFF_TW = NBUF * BUF, OFF_BAR = OFF_TW + TWB;
+  static constexpr int SMEM_BYTES = OFF_BAR + 128 + 1024;
+  static void fill_twiddles(float* out) {
+    constexpr double pi2 = 6.283185307179586476925286766559, sgn = INV ? 1.0 : -1.0;
+    auto set = [&](u32 at, u32 p, u32 e, u32 mod, double scale) {
+      const double x = pi2 * (double)(e % mod) / (double)mod;
+      out[at * 4 + p] = (float)(scale * std::cos(x));
+      out[at * 4 + 2 + p] = (float)(scale * sgn * std::sin(x));
+    };
+    for (u32 p = 0; p < 2; ++p) {
+      for (u32 warp = 0; warp < 2; ++warp)
+        for (u32 mh = 0; mh < 4; ++mh)
+          for (u32 lane = 0; lane < 32; ++lane) {
+            const XY a = p1((lane & 3u) << 1 | p, mh & 1u, 0, warp);
+            set((warp * 4 + mh) * 32 + lane, p, ((lane >> 2) + 8 * (mh >> 1)) * (8 * a.x + a.y), 2048, 1.0);
+          }
+      for (u32 k1 = 0; k1 < 16; ++k1) set(256 + k1, p, k1, 2048, 1.0);
+      for (u32 n3 = 1; n3 < 8; ++n3)
+        for (u32 mt = 0; mt < 2; ++mt)
+          for (u32 g = 0; g < 8; ++g) set(272 + ((n3 - 1) * 2 + mt) * 8 + g, p, (g + 8 * mt) * n3, 128, 0.125);
+    }
+  }
+  static void fill_fragments(uint32_t* out) { MmaPass<256, kRR, false, INV>::fill_fragments(out); }
+  template <class A>
+  static __device__ __forceinline__ void setup(const A&, uint8_t*, int) {}
+  using M = MmaPass<256, kRR, false, INV>;
+
+  template <class A>
+  static __device__ __forceinline__ void run(const A&, const State& st, u32 sb, u32 tws, int t, u32,
+                                             const Sync<T>&) {
+    const u32 lane = t & 31, warp = (t >> 5) & 1u, g = lane >> 2;
+    const int bar = 8 + (t >> 6);
+    sb += (t >> 6) * 8192;
+    u32 x[8][4];
+    {
+      const u32 lb = sb + load1_t(lane, warp), sp = sb + store1_t(lane, warp);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) Mma4096<INV>::get(lb, load1_r(j >> 2, j & 3), x[j]);
+      __syncwarp();
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        P2 cr[2], ci[2];
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt) {
+          const float4 f = lds128f(tws + ((warp * 4 + mt * 2 + h) * 32 + lane) * 16);
+          cr[mt] = pack2(f.x, f.y);
+          ci[mt] = pack2(f.z, f.w);
+        }
+        u32 o[2][2][4];
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+          P2 re[2], im[2];
+          M::unit(st, x[4 * h][w], x[4 * h + 1][w], x[4 * h + 2][w], x[4 * h + 3][w], re, im);
+#pragma unroll
+          for (int mt = 0; mt < 2; ++mt) {
+            cmulv(re[mt], im[mt], cr[mt], ci[mt]);
+            if (w < 3) {
+              const float4 f = lds128f(tws + (256 + g + 8 * mt) * 16);
+              cmulv(cr[mt], ci[mt], pack2(f.x, f.y), pack2(f.z, f.w));
+            }
+            M::to_words(re[mt], im[mt], o[mt][0][w], o[mt][1][w]);
+          }
+        }
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+          for (int p = 0; p < 2; ++p) M::put(sp, store1_r(mt, p, h), o[mt][p]);
+      }
+    }
+    col_bar<64>(bar);
+    {
+      const u32 lb = sb + load2_t(lane, warp), sp = sb + store2_t(lane, warp);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) Mma4096<INV>::get(lb, load2_r(j >> 2, j & 3), x[j]);
+      col_bar<64>(bar);
+#pragma unroll
+      for (int mt = 0; mt < 2; ++mt) {
+        P2 zr[8], zi[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const int j = u & 4, w = u & 3;  // n3 = w + 4 h
+          float d[4];
+          mma16816<true>(d, st.a[mt][0], x[j][w], x[j + 1][w]);
+          mma16816<false>(d, st.a[mt][1], x[j + 2][w], x[j + 3][w]);
+          zr[u] = pack2(d[0], d[1]);
+          zi[u] = pack2(d[2], d[3]);
+          if (u == 0) {
+            zr[0] = zr[0] * num<P2>(0.125f);
+            zi[0] = zi[0] * num<P2>(0.125f);
+          } else {
+            const float4 f = lds128f(tws + (272 + ((u - 1) * 2 + mt) * 8 + g) * 16);
+            cmulv(zr[u], zi[u], pack2(f.x, f.y), pack2(f.z, f.w));
+          }
+        }
+        Dft<8, INV, P2>::run(zr, zi);
+#pragma unroll
+        for (int k3 = 0; k3 < 8; ++k3) {
+          u32 w0, w1;
+          M::to_words(zr[k3], zi[k3], w0, w1);
+          const u32 d = store2_r(mt, k3);
+          tile::sts64((sp ^ (d & XM)) + (d & ~XM), make_float2(__uint_as_float(w0), __uint_as_float(w1)));
+        }
       }
     }
   }

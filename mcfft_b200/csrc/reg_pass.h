@@ -3,7 +3,7 @@
 #pragma once
 #include "fft_mma.cuh"
 #include "fft_reg.cuh"
-#include "fft_reg4096.cuh"
+#include "fft_rows.cuh"
 #include "tile_pass.h"
 
 namespace mcfft {
@@ -61,11 +61,10 @@ TileKernel make_mma() {
   return k;
 }
 
-// 4096-point rows (fft_reg4096.cuh).
-inline TileKernel make_mma4096() {
-  using P = reg::Mma4096<false>;
-  using Q = reg::Mma4096<true>;
-  TileKernel k{reinterpret_cast<const void*>(&reg::fft_reg<P>), 4096, 16, 1, false, false, P::THREADS,
+// Rows of 2048 and 4096 points (fft_rows.cuh), plain form.
+template <class P, class Q>
+TileKernel make_mma_rows() {
+  TileKernel k{reinterpret_cast<const void*>(&reg::fft_reg<P>), P::L, P::R, P::C, false, false, P::THREADS,
                P::SMEM_BYTES, 0, P::TP, true};
   k.fn_inv = reinterpret_cast<const void*>(&reg::fft_reg<Q>);
   k.reg_kind = reg::kRR;
@@ -77,6 +76,7 @@ inline TileKernel make_mma4096() {
   k.fill_frag[1] = &Q::fill_fragments;
   return k;
 }
+// 4096-point rows, FP32 exchange.
 template <bool IN16>
 TileKernel make_reg4096() {
   using P = reg::Reg4096<IN16, false>;

@@ -33,7 +33,8 @@ const std::vector<TileKernel>& reg_registry_plain() {
       make_mma<256, reg::kRR, false, 4096>(),
       make_mma<512, reg::kRR, false, 4096>(),
       make_mma<1024, reg::kRR, false, 4096>(),
-      make_mma4096()};
+      make_mma_rows<reg::Mma4096<false>, reg::Mma4096<true>>(),
+      make_mma_rows<reg::Mma2048<false>, reg::Mma2048<true>>()};
   return v;
 }
 

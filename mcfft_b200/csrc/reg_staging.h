@@ -70,29 +70,37 @@ inline layout::Staging reg_col_staging(int L, int C, int elem, bool swizzled, co
   return s;
 }
 
-// 4096-point rows: plain (swizzled) 128-byte rows of 32 points, row 16 (p /
-// 32 mod 8) + p / 256; FP32 exchange: natural order.
-inline layout::Staging reg_4096_staging(int elem, bool mma, int64_t sc, int64_t so, int64_t ncols,
-                                        int64_t nouter) {
+// Rows of 2048 and 4096 points.  Plain: swizzled 128-byte rows of 32 points,
+// within a transform row 16 (p / 32 mod B) + p / (32 B) with B = L / 512 (the
+// 2048-point output: natural); FP32 exchange: natural order, no swizzle.
+inline layout::Staging reg_rows_staging(const RegShape& k, bool out, int elem, int64_t sc, int64_t so,
+                                        int64_t ncols, int64_t nouter) {
   layout::Staging s;
   s.kind = layout::ROW;
-  s.L = 4096;
-  s.C = 1;
+  s.L = k.L;
+  s.C = k.C;
   s.elem = elem;
-  s.E = mma ? 32 : 256;
+  s.E = k.mma ? 32 : 256;
   s.row_bytes = s.E * elem;
-  s.swz = mma ? 7 : 0;
+  s.swz = k.mma ? 7 : 0;
+  const int B = k.L / 512;
   reg_add_dim(&s, s.E, s.E, 1, 0, 0);
-  reg_add_dim(&s, 16, 16, 256, 0, 0);
-  if (mma) reg_add_dim(&s, 8, 8, 32, 0, 0);
-  reg_add_dim(&s, ncols, 1, sc, 1, 0);
+  if (!k.mma) {
+    reg_add_dim(&s, k.L / 256, k.L / 256, 256, 0, 0);
+  } else if (out && k.L == 2048) {
+    reg_add_dim(&s, 64, 64, 32, 0, 0);
+  } else {
+    reg_add_dim(&s, 16, 16, 32 * B, 0, 0);
+    reg_add_dim(&s, B, B, 32, 0, 0);
+  }
+  reg_add_dim(&s, ncols, k.C, sc, k.C, 0);
   if (nouter > 1) reg_add_dim(&s, nouter, 1, so, 0, 1);
   return s;
 }
 
 inline layout::Staging reg_staging_in(const RegShape& k, layout::Kind ik, int elem, int64_t sp, int64_t sc,
                                       int64_t so, int64_t ncols, int64_t nouter) {
-  if (k.L == 4096) return reg_4096_staging(elem, k.mma, sc, so, ncols, nouter);
+  if (k.L > 1024) return reg_rows_staging(k, false, elem, sc, so, ncols, nouter);
   if (ik == layout::ROW) return reg_row_staging(k.L, k.C, elem, k.mma, sc, so, ncols, nouter);
   if (k.mma) {  // rows [v][n1], n = n1 (L / 16) + v
     const int dig[2] = {16, k.L / 16};
@@ -107,7 +115,7 @@ inline layout::Staging reg_staging_in(const RegShape& k, layout::Kind ik, int el
 
 inline layout::Staging reg_staging_out(const RegShape& k, layout::Kind ik, layout::Kind ok, int elem,
                                        int64_t sp, int64_t sc, int64_t so, int64_t ncols, int64_t nouter) {
-  if (k.L == 4096) return reg_4096_staging(elem, k.mma, sc, so, ncols, nouter);
+  if (k.L > 1024) return reg_rows_staging(k, true, elem, sc, so, ncols, nouter);
   if (ok == layout::ROW) return reg_row_staging(k.L, k.C, elem, k.mma, sc, so, ncols, nouter);
   if (k.mma) {  // rows [k1][k3][k2], X[k1 + 16 k2 + 256 k3]
     const int dig[3] = {16, k.R, 16};

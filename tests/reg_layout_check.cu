@@ -11,7 +11,7 @@
 #include <vector>
 
 #include "../mcfft_b200/csrc/fft_mma.cuh"
-#include "../mcfft_b200/csrc/fft_reg4096.cuh"
+#include "../mcfft_b200/csrc/fft_rows.cuh"
 #include "../mcfft_b200/csrc/reg_staging.h"
 
 using namespace mcfft;
@@ -385,6 +385,88 @@ static void check_mma4096() {
   printf("%s 4096-point rows, plain\n", g_bad == bad0 ? "ok" : "FAULT");
 }
 
+// 2048-point rows, plain form.
+static void check_mma2048() {
+  using M = Mma2048<false>;
+  const int bad0 = g_bad;
+  const RegShape sh{2048, 8, 8, 0, true};
+  const auto tin = tma_place(reg_staging_in(sh, layout::ROW, 4, 1, 2048, 0, 8, 1), true);
+  const auto tout = tma_place(reg_staging_out(sh, layout::ROW, layout::ROW, 4, 1, 2048, 0, 8, 1), true);
+  auto at = [&](uint32_t t, uint32_t r) { return (t ^ (r & M::XM)) + (r & ~M::XM); };
+  int excess = 0;
+  for (uint32_t c = 0; c < 8; ++c) {
+    std::vector<int> slot(2048, -1), out(2048, 0), seen(2048, 0);
+    for (uint32_t w = 0; w < 2; ++w) {
+      std::set<uint32_t> rd, wr;
+      for (uint32_t j = 0; j < 8; ++j) {
+        std::vector<uint32_t> la;
+        for (uint32_t l = 0; l < 32; ++l) {
+          const uint32_t x = at(M::load1_t(l, w), M::load1_r(j >> 2, j & 3));
+          CHECK(x % 16 == 0 && x + 16 <= 8192, "access %u", x);
+          for (uint32_t u = 0; u < 4 && x + 16 <= 8192; ++u) {
+            const auto a = M::p1(l >> 2, j >> 2, u, w);
+            const uint32_t pos = ((l & 3) + 4 * (j & 3)) * 128 + a.x * 8 + a.y;
+            CHECK(tin[pos * 8 + c] == c * 8192 + x + 4 * u, "point %u", pos);
+            ++seen[pos];
+            rd.insert(x + 4 * u);
+          }
+          la.push_back(x);
+        }
+        excess += wavefronts(la, 16) - 4;
+      }
+      for (uint32_t e = 0; e < 8; ++e) {
+        std::vector<uint32_t> sa;
+        for (uint32_t l = 0; l < 32; ++l) {
+          const uint32_t x = at(M::store1_t(l, w), M::store1_r(e & 1, (e >> 1) & 1, e >> 2));
+          CHECK(x % 16 == 0 && x + 16 <= 8192, "access %u", x);
+          for (uint32_t u = 0; u < 4 && x + 16 <= 8192; ++u) {
+            const auto a = M::p1((l & 3) << 1 | ((e >> 1) & 1), e >> 2, u, w);
+            CHECK(slot[x / 4 + u] < 0, "slot written twice");
+            slot[x / 4 + u] = (int)(((l >> 2) + 8 * (e & 1)) * 128 + a.x * 8 + a.y);
+            wr.insert(x + 4 * u);
+          }
+          sa.push_back(x);
+        }
+        excess += wavefronts(sa, 16) - 4;
+      }
+      CHECK(rd == wr, "phase 1 leaves its slots");
+    }
+    for (uint32_t w = 0; w < 2; ++w) {
+      for (uint32_t j = 0; j < 8; ++j) {
+        std::vector<uint32_t> la;
+        for (uint32_t l = 0; l < 32; ++l) {
+          const uint32_t x = at(M::load2_t(l, w), M::load2_r(j >> 2, j & 3));
+          CHECK(x % 16 == 0 && x + 16 <= 8192, "access %u", x);
+          for (uint32_t u = 0; u < 4 && x + 16 <= 8192; ++u) {
+            const auto a = M::p2(l >> 2, j >> 2, u, w);
+            CHECK(slot[x / 4 + u] == (int)(a.x * 128 + ((l & 3) + 4 * (j & 3)) * 8 + a.y), "phase 2 load");
+          }
+          la.push_back(x);
+        }
+        excess += wavefronts(la, 16) - 4;
+      }
+      for (uint32_t e = 0; e < 16; ++e) {
+        std::vector<uint32_t> sa;
+        for (uint32_t l = 0; l < 32; ++l) {
+          const uint32_t x = at(M::store2_t(l, w), M::store2_r(e & 1, e >> 1));
+          CHECK(x % 8 == 0 && x + 8 <= 8192, "access %u", x);
+          for (uint32_t p = 0; p < 2 && x + 8 <= 8192; ++p) {
+            const auto a = M::p2((l & 3) << 1 | p, 0, 0, w);
+            const uint32_t pos = a.x + 16 * ((l >> 2) + 8 * (e & 1)) + 256 * (e >> 1);
+            CHECK(tout[pos * 8 + c] == c * 8192 + x + 4 * p, "output %u", pos);
+            ++out[pos];
+          }
+          sa.push_back(x);
+        }
+        excess += wavefronts(sa, 8) - 2;
+      }
+    }
+    for (int i = 0; i < 2048; ++i) CHECK(seen[i] == 1 && out[i] == 1, "point %d: %d loads, %d stores", i, seen[i], out[i]);
+  }
+  CHECK(excess == 0, "%d wavefronts of bank conflicts", excess);
+  printf("%s 2048-point rows, plain\n", g_bad == bad0 ? "ok" : "FAULT");
+}
+
 // 4096-point rows, FP32 exchange.
 static void check_reg4096() {
   using M = Reg4096<false, false>;
@@ -437,6 +519,7 @@ static void check_reg4096() {
 
 int main() {
   check_mma4096();
+  check_mma2048();
   check_reg4096();
   W(256, kRR, false), W(512, kRR, false), W(1024, kRR, false);
   WS(256), WS(512), WS(1024);

@@ -84,3 +84,10 @@ def test_four_step(n, batch, form, direction):
                                          ((1024, 64), 150), ((64, 128, 32), 7), ((256, 64, 16), 11)])
 def test_columns(shape, batch, form):
     _check(shape, batch, form, mc.FORWARD)
+
+
+@pytest.mark.parametrize("direction", [mc.FORWARD, mc.INVERSE])
+@pytest.mark.parametrize("shape,batch", [((2048,), 1), ((2048,), 8), ((2048,), 5001), ((64, 2048), 9),
+                                         ((2048, 128), 5)])
+def test_rows_2048(shape, batch, direction):
+    _check(shape, batch, "plain", direction)
