@@ -261,6 +261,7 @@ struct MmaPass {
   static constexpr int SMEM_BYTES = OFF_BAR + 128 + 1024;
   static_assert(SMEM_BYTES <= 232448, "shared memory budget");
 
+  static constexpr int TABB = OFF_BAR - OFF_TW;  // all tables
   using State = MmaFrags;
 
   // DFT-16 of the unit whose operand slots are b0 .. b3: pairs re[mt], im[mt].

@@ -140,6 +140,7 @@ struct RegPass {
   static constexpr int THREADS = NG * T + (BIG ? 128 : 32), MINB = BIG ? 1 : 3;
   static constexpr int OFF_TW = NBUF * BUF;
   static constexpr int OFF_BAR = OFF_TW + TWB;
+  static constexpr int TABB = TWB;  // all tables
   static constexpr int SMEM_BYTES = OFF_BAR + 128 + 1024;
   static_assert(SMEM_BYTES <= 232448, "shared memory budget");
 

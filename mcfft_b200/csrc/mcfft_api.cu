@@ -21,10 +21,11 @@
 // embedding) are generated in FP64 on the GPU at plan time for both
 // directions; the plain form's four-step twiddles and the radix-2 twiddles
 // of 8192-point passes are instead computed in the kernel from their exact
-// angle.  A plan of several transform groups (mcfftPlanCreateBatch) whose
-// passes all run on tile kernels the batch kernel holds executes as one
-// launch of the persistent batch kernel (fft_queue.cuh) over a queue of
-// (pass, tile) items built here; otherwise one launch per pass.
+// angle.  A plan of several transform groups (mcfftPlanCreateBatch) executes
+// as one launch of a persistent kernel over a queue of (pass, tile) items
+// built here: plain plans of register passes on reg_queue.cuh, else, if every
+// pass runs on a tile kernel the batch kernel (fft_queue.cuh) holds, on that;
+// otherwise one launch per pass.
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -42,6 +43,7 @@
 #include "host_schedule.h"
 #include "queue_order.h"
 #include "reg_pass.h"
+#include "reg_queue.h"
 #include "tile_pass.h"
 
 namespace mcfft {
@@ -114,6 +116,11 @@ struct Queue {
   const void* fn = nullptr;
   int smem = 0;
   bool fused = false;
+  // Every pass is a register pass: the one-launch kernel of reg_queue.cuh
+  // (rargs) instead of the batch kernel.
+  bool reg = false, resident = false;
+  RArgs* rargs = nullptr;
+  RItem* ritems = nullptr;
   // Fault injection for the failure-detection tests (MCFFT_INJECT_STALL at
   // plan time): every dependent pass waits for a producer count that can
   // never be reached, so its tiles time out on the device and the exec
@@ -145,6 +152,8 @@ struct mcfftPlan_st {
   // The plan is meant for the batch queue (several transform groups, or
   // MCFFT_QUEUE=1): its passes take only tile shapes the batch kernel holds.
   bool queue_planned = false;
+  // The same for the one-launch kernel on the register passes.
+  bool reg_queue = false;
   // A group the batch queue cannot run (three-pass 1D lengths).
   bool no_queue = false;
   // An indexed transform group (per-transform offsets), which only the
@@ -414,26 +423,37 @@ mcfftResult add_tile_pass(mcfftPlan p, const PassSpec& s, int only_tile_points =
   const TileKernel* k = nullptr;
   std::vector<int32_t> in_tab, out_tab;
   const bool indexed = s.gather || !s.in_idx.empty() || !s.out_idx.empty();
-  // Register kernels (fft_reg.cuh) first, for the lengths of two phases (64 ..
-  // 1024): faster than the tcgen05 tiles in every case measured (split form
-  // 1.33x .. 1.39x on four-step, 2D and 3D transforms, plain 1.04x .. 1.13x).
-  // Passes of the batch queue, longer columns and the plain form's 8K-point
-  // tiles (small batches) take the tcgen05 tiles.
-  const int small = small_tiles(p, s) && !only_tile_points ? 4096 : 0;
+  // Register kernels (fft_reg.cuh, fft_mma.cuh, fft_rows.cuh) first: faster
+  // than the tcgen05 tiles in every case measured (split form 1.33x .. 1.39x
+  // on four-step, 2D and 3D transforms, plain 1.04x .. 1.13x).  Passes of the
+  // batch queue, longer columns and the plain form's 8K-point tiles (small
+  // batches) take the tcgen05 tiles; those of the one-launch kernel are
+  // register passes or none.
+  const int small = small_tiles(p, s) && !only_tile_points && !p->reg_queue ? 4096 : 0;
   for (int oi = small ? -1 : 0; oi < 2 && !k; ++oi) {
-    if (p->queue_planned || indexed) break;
+    if (!p->reg_queue && (p->queue_planned || indexed)) break;
     const TileKernel* cand = find_reg_kernel((int)s.L, ik, ok, s.posttw, p->split,
                                              oi < 0 ? small : order[oi], s.in_f16 != 0);
     if (!cand || (s.ncols + cand->C - 1) / cand->C * s.nouter >= (int64_t(1) << 31)) continue;
+    if (p->reg_queue && reg_queue_variant(*cand) < 0) continue;
     layout::Staging si, so;
-    reg_stagings(*cand, ik, ok, in_elem, out_elem, s.in_sp, s.in_sc, s.in_so, s.out_sp, s.out_sc,
-                 s.out_so, s.ncols, s.nouter, &si, &so);
+    if (s.gather) {
+      if (!reg_gather_staging(*cand, false, in_elem, s.in_idx, &si, &in_tab) ||
+          !reg_gather_staging(*cand, true, out_elem, s.out_idx, &so, &out_tab))
+        continue;
+    } else {
+      reg_stagings(*cand, ik, ok, in_elem, out_elem, s.in_sp, s.in_sc, s.in_so, s.out_sp, s.out_sc,
+                   s.out_so, s.ncols, s.nouter, &si, &so);
+      if (!s.in_idx.empty() && !index_outer(&si, s.in_idx, &in_tab)) continue;
+      if (!s.out_idx.empty() && !index_outer(&so, s.out_idx, &out_tab)) continue;
+    }
     if (si.ndims < 3 || si.ndims > 5 || so.ndims < 3 || so.ndims > 5) continue;
     if (!tile_check_encode(si, p->status) || !tile_check_encode(so, p->status)) continue;
     tp.lay.in = si;
     tp.lay.out = so;
     k = cand;
   }
+  if (p->reg_queue && !k) return MCFFT_UNSUPPORTED_SIZE;
   for (int oi = 0; oi < 2 && !k; ++oi) {
     const TileKernel* cand =
         find_tile_kernel((int)s.L, s.posttw, p->split, order[oi], s.in_f16 != 0);
@@ -663,7 +683,7 @@ void wisdom_put(const std::string& key, int tile_points) {
 // scratch buffers and keeps the faster (by more than 3 %), which is then
 // recorded.  MCFFT_AUTOTUNE=0 keeps the default shapes.
 mcfftResult autotune_group(mcfftPlan p, size_t first, int64_t points) {
-  if (p->split) return MCFFT_SUCCESS;
+  if (p->split || p->reg_queue) return MCFFT_SUCCESS;
   if (const char* e = std::getenv("MCFFT_AUTOTUNE"))
     if (std::atoi(e) == 0) return MCFFT_SUCCESS;
   const std::string gk = gpu_key(p);
@@ -725,7 +745,7 @@ mcfftResult add_pass(mcfftPlan p, const PassSpec& s) {
     mcfftResult tr = add_tile_pass(p, s);
     if (tr != MCFFT_UNSUPPORTED_SIZE) return tr;
     // the direct-load kernels address only affine layouts
-    if (s.gather || !s.in_idx.empty() || !s.out_idx.empty()) return tr;
+    if (p->reg_queue || s.gather || !s.in_idx.empty() || !s.out_idx.empty()) return tr;
   }
   const PassKernel* k =
       pick_pass_kernel((int)s.L, s.colfast, s.posttw, p->split, s.ncols, tile_points_env());
@@ -835,6 +855,11 @@ int64_t max_four_column(const mcfftPlan p) { return p->split ? kMaxTilePass / 2 
 // pairs run a direct-load pass (2^26: 2.68 ms against 0.42 ms).
 int default_lg1(const mcfftPlan p, int64_t n) {
   if (n <= max_one_pass(p)) return kOnePass;
+  // In the one-launch kernel columns of 256 points run on the tensor cores, of
+  // 128 they do not: 2^14 x 4096 in 228 us as 128 x 128, 2^15 x 2048 in 213 us
+  // as 128 x 256; as pass launches 213 and 215, with 256-point columns 191 and
+  // 194.
+  if (p->reg_queue) return ilog2(n) < 14 ? ilog2(n) / 2 : std::max(8, ilog2(n) / 2);
   if (n >= (p->split ? (int64_t(1) << 23) : (int64_t(1) << 24))) return kThreePass;
   return ilog2(n) / 2;
 }
@@ -1193,7 +1218,7 @@ int tune_fourstep(mcfftPlan p, int64_t n, int64_t batch, int64_t in_off, int64_t
 mcfftResult build_group(mcfftPlan p, int ndim, const int64_t* dims, int64_t batch,
                         int64_t in_off, int64_t out_off, int* scale_log2) {
   const size_t first = p->passes.size();
-  p->fs_lg1 = ndim == 1 ? tune_fourstep(p, dims[0], batch, in_off, out_off) : 0;
+  p->fs_lg1 = ndim == 1 && !p->reg_queue ? tune_fourstep(p, dims[0], batch, in_off, out_off) : 0;
   mcfftResult r = build_group_passes(p, ndim, dims, batch, in_off, out_off, scale_log2);
   if (!r && ndim == 1 && first == 0 && p->passes.size() >= 2)
     p->info.fourstep_n1 = p->passes[0].spec.L;
@@ -1237,7 +1262,7 @@ mcfftResult build_indexed_group(mcfftPlan p, int ndim, const int64_t* dims,
       sp.gather = true;
       r = add_pass(p, sp);
     } else if (n <= kMaxSinglePass * kMaxSinglePass) {
-      const int lg = ilog2(n), lg1 = lg / 2;
+      const int lg1 = p->reg_queue ? default_lg1(p, n) : ilog2(n) / 2;
       const int64_t n1 = int64_t(1) << lg1, n2 = n >> lg1;
       if (n1 < 16 || n2 < 16 || n1 > kMaxSinglePass || n2 > kMaxSinglePass)
         return MCFFT_UNSUPPORTED_SIZE;
@@ -1403,6 +1428,21 @@ const FusedKernel* fused_for(mcfftPlan p) {
   return find_fused(p->split, v1, v2);
 }
 
+// The passes of a plan as the queue order sees them.
+std::vector<QOrderPass> queue_passes(const mcfftPlan p) {
+  std::vector<QOrderPass> qo(p->passes.size());
+  for (size_t i = 0; i < qo.size(); ++i) {
+    const Pass& ps = p->passes[i];
+    qo[i].ntiles = ps.tp.args.ntiles;
+    qo[i].col_blocks = ps.tp.args.col_blocks;
+    qo[i].sig_mul = ps.sig_mul;
+    qo[i].sig_div = ps.sig_div;
+    qo[i].keys = ps.level > 0 ? ps.keys : 0;
+    qo[i].grp = ps.grp;
+  }
+  return qo;
+}
+
 // Builds the batch queue (every pass of the plan in one persistent launch)
 // for plans of several transform groups (uneven batches) -- or any plan
 // with MCFFT_QUEUE=1; MCFFT_QUEUE=0 disables it -- when every pass runs on
@@ -1457,19 +1497,9 @@ mcfftResult build_queue(mcfftPlan p) {
   // consecutive items switch pass)
   int64_t QC = fk ? 2 : 16;
   if (const char* e = std::getenv("MCFFT_QUEUE_CHUNK")) QC = std::max<int64_t>(1, std::atoll(e));
-  std::vector<QOrderPass> qo(np);
-  for (size_t i = 0; i < np; ++i) {
-    const Pass& ps = p->passes[i];
-    qo[i].ntiles = ps.tp.args.ntiles;
-    qo[i].col_blocks = ps.tp.args.col_blocks;
-    qo[i].sig_mul = ps.sig_mul;
-    qo[i].sig_div = ps.sig_div;
-    qo[i].keys = ps.level > 0 ? ps.keys : 0;
-    qo[i].grp = ps.grp;
-  }
   int64_t QLAG = 0;  // lag between a key's completion and its readers (0: QC)
   if (const char* e = std::getenv("MCFFT_QUEUE_LAG")) QLAG = std::max<int64_t>(0, std::atoll(e));
-  const std::vector<QOrderItem> order = queue_order(qo, G, QC, QLAG);
+  const std::vector<QOrderItem> order = queue_order(queue_passes(p), G, QC, QLAG);
   if (order.empty()) return MCFFT_SUCCESS;  // no consistent order: pass by pass
   std::vector<QItem> items(order.size());
   for (size_t i = 0; i < order.size(); ++i) items[i] = {order[i].pass, order[i].tile};
@@ -1509,6 +1539,119 @@ mcfftResult build_queue(mcfftPlan p) {
   if (!q.args) return MCFFT_ALLOC_FAILED;
   q.stall = std::getenv("MCFFT_INJECT_STALL") != nullptr;
   q.on = true;
+  return MCFFT_SUCCESS;
+}
+
+// The queue of a plan for the one-launch kernel on the register passes
+// (reg_queue.cuh), in the same order.  MCFFT_UNSUPPORTED_SIZE: the caller
+// plans for the batch kernel instead.  Chunks of 16 first-pass tiles per CTA:
+// a batch of 4096 1D transforms of 2^8 .. 2^16 points and 64 of 128 .. 512
+// points a side takes 241 us (14 runs of one pass per CTA), in chunks of 8
+// 242 .. 246, of 4 249, of 32 240; the batch kernel takes 350 us.
+mcfftResult build_reg_queue(mcfftPlan p) {
+  const size_t np = p->passes.size();
+  if (np > (size_t)kRegQueueMaxPasses || p->no_queue) return MCFFT_UNSUPPORTED_SIZE;
+  int64_t tabs = 0, nc = 0;
+  for (const auto& ps : p->passes) {
+    if (!ps.tiled || reg_queue_variant(*ps.tp.k) < 0 || (ps.level > 0 && ps.keys < 1) ||
+        ps.sig_div > INT32_MAX || ps.sig_mul > INT32_MAX)
+      return MCFFT_UNSUPPORTED_SIZE;
+    tabs += (ps.tp.k->tab_bytes + 127) / 128 * 128;
+  }
+  const int64_t G = reg_queue_max_grid(p->sms);
+  if (G <= 0) return MCFFT_UNSUPPORTED_SIZE;
+  Queue& q = p->q;
+  q.resident = tabs <= reg::QueueShape::TAB_BYTES;
+  int64_t QC = 16, lag = 0;
+  if (const char* e = std::getenv("MCFFT_QUEUE_CHUNK")) QC = std::max<int64_t>(1, std::atoll(e));
+  if (const char* e = std::getenv("MCFFT_QUEUE_LAG")) lag = std::max<int64_t>(0, std::atoll(e));
+  const std::vector<QOrderItem> order = queue_order(queue_passes(p), G, QC, lag);
+  if (order.empty() || order.size() > (size_t)INT32_MAX) return MCFFT_UNSUPPORTED_SIZE;
+  q.wait_base.assign(np, -1);
+  q.sig_base.assign(np, -1);
+  for (size_t i = 0; i < np; ++i)
+    if (p->passes[i].level > 0) {
+      q.wait_base[i] = (int)nc;
+      q.sig_base[i - 1] = (int)nc;
+      nc += p->passes[i].keys;
+    }
+  std::vector<RItem> items(order.size());
+  for (size_t i = 0; i < order.size(); ++i) items[i] = {order[i].pass, order[i].tile};
+  RItem* d = nullptr;
+  mcfftResult r = plan_alloc(p, &d, items.size() * sizeof(RItem));
+  if (!r) r = plan_alloc(p, &q.counters, (size_t)(nc + 1) * sizeof(int));
+  if (r) return r;
+  if (cudaMemcpy(d, items.data(), items.size() * sizeof(RItem), cudaMemcpyHostToDevice) != cudaSuccess ||
+      cudaMemset(q.counters, 0, (size_t)(nc + 1) * sizeof(int)) != cudaSuccess)
+    return MCFFT_CUDA_ERROR;
+  q.ritems = d;
+  q.nitems = (int64_t)items.size();
+  q.ncounters = nc;
+  q.grid = (int)std::min<int64_t>(G, q.nitems);
+  q.rargs = new (std::nothrow) RArgs();
+  if (!q.rargs) return MCFFT_ALLOC_FAILED;
+  q.stall = std::getenv("MCFFT_INJECT_STALL") != nullptr;
+  q.reg = q.on = true;
+  if (std::getenv("MCFFT_DEBUG_PLAN")) {
+    int64_t runs = 0;
+    for (int64_t i = 0; i < q.nitems; ++i)
+      runs += i < q.grid || items[i].pass != items[i - q.grid].pass ? 1 : 0;
+    fprintf(stderr, "[mcfft] one launch: %zu passes, %zu items on %d CTAs, %.1f runs per CTA, tables %s\n", np,
+            items.size(), q.grid, (double)runs / q.grid, q.resident ? "resident" : "reloaded");
+  }
+  return MCFFT_SUCCESS;
+}
+
+mcfftResult exec_reg_queue(mcfftPlan p, const void* in, void* out, int dir, cudaStream_t st) {
+  Queue& q = p->q;
+  RArgs& A = *q.rargs;
+  A.items = q.ritems;
+  A.nitems = (uint32_t)q.nitems;
+  A.npass = (int)p->passes.size();
+  A.counters = q.counters;
+  A.ncounters = (int)q.ncounters;
+  A.resident = q.resident;
+  A.status = p->status;
+  A.bmat = p->bsw64[dir];  // any 2 KB; the fragments if a pass uses them
+  auto base = [&](int b) -> char* {
+    return b == kUserIn ? (char*)const_cast<void*>(in) : b == kUserOut ? (char*)out : (char*)p->scratch;
+  };
+  uint32_t off = 0;
+  for (size_t i = 0; i < p->passes.size(); ++i) {
+    const Pass& ps = p->passes[i];
+    RPass& Q = A.pass[i];
+    const int ib = ps.in_f16 ? 4 : 8, ob = ps.out_f16 ? 4 : 8;
+    if (!fill_rpass(ps.tp, dir, base(ps.in_buf) + ps.in_off * ib, base(ps.out_buf) + ps.out_off * ob, &Q))
+      return MCFFT_CUDA_ERROR;
+    if (ps.tp.k->mma) A.bmat = ps.tp.bmat[dir];
+    if (ps.in_tab || ps.out_tab) {
+      const bool g = ps.spec.gather;
+      (g ? Q.in_gtab : Q.in_otab) = ps.in_tab;
+      (g ? Q.out_gtab : Q.out_otab) = ps.out_tab;
+      Q.g_cols = (uint32_t)ps.spec.ncols;
+      Q.g_tile = (uint32_t)ps.tp.k->C;
+      Q.g_bytes = (uint32_t)ps.tp.k->L * 4;
+    }
+    Q.tw_off = off;
+    off += (uint32_t)(ps.tp.k->tab_bytes + 127) / 128 * 128;
+    Q.wait_base = q.wait_base[i];
+    Q.wait_count = q.stall && Q.wait_base >= 0 ? INT32_MAX : ps.wait_count;
+    Q.sig_base = q.sig_base[i];
+    Q.sig_mul = (int32_t)ps.sig_mul;
+    Q.sig_div = (int32_t)ps.sig_div;
+    Q.sig_kmax = q.sig_base[i] >= 0 && i + 1 < p->passes.size() ? (int32_t)p->passes[i + 1].keys - 1 : 0;
+  }
+  cudaError_t e = launch_reg_queue(A, q.grid, dir, st);
+  if (e == cudaSuccess && std::getenv("MCFFT_DEBUG_SYNC")) {
+    e = cudaStreamSynchronize(st);
+    fprintf(stderr, "[mcfft] one launch: %d passes, %lld items, grid %d: %s\n", A.npass, (long long)q.nitems,
+            q.grid, cudaGetErrorString(e));
+  }
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return MCFFT_CUDA_ERROR;
+  }
+  p->last_stream = st;
   return MCFFT_SUCCESS;
 }
 
@@ -1560,8 +1703,9 @@ mcfftResult exec_queue(mcfftPlan p, const void* in, void* out, int dir, cudaStre
 
 mcfftResult plan_finish(mcfftPlan p, mcfftPlan* out) {
   mcfftResult r = MCFFT_SUCCESS;
-  if (p->scratch_bytes) r = plan_alloc(p, &p->scratch, p->scratch_bytes);
-  if (!r) r = build_queue(p);
+  if (p->reg_queue) r = build_reg_queue(p);
+  if (!r && p->scratch_bytes) r = plan_alloc(p, &p->scratch, p->scratch_bytes);
+  if (!r && !p->reg_queue) r = build_queue(p);
   if (!r && p->indexed && !p->q.on) r = MCFFT_UNSUPPORTED_SIZE;
   if (!r) r = cuda_fail(cudaDeviceSynchronize());
   if (r) {
@@ -1670,7 +1814,7 @@ int in_elem(const mcfftPlan p, const Pass& ps) { return p->split ? (ps.in_f16 ? 
 int out_elem(const mcfftPlan p, const Pass& ps) { return p->split ? (ps.out_f16 ? 4 : 8) : 4; }
 
 mcfftResult exec_launches(mcfftPlan p, const void* in, void* out, int dir, cudaStream_t st) {
-  if (p->q.on) return exec_queue(p, in, out, dir, st);
+  if (p->q.on) return p->q.reg ? exec_reg_queue(p, in, out, dir, st) : exec_queue(p, in, out, dir, st);
   for (size_t i = 0; i < p->passes.size(); ++i) {
     const Pass& ps = p->passes[i];
     auto base = [&](int b) -> char* {
@@ -1818,8 +1962,11 @@ namespace {
 // (indexed where its transforms are not contiguous and in order; *indexed
 // tells whether any was); else one group per run of consecutive
 // descriptors of one shape whose data follow each other in both buffers.
+// reg: for the one-launch kernel on the register passes, which takes plans of
+// several groups whose passes are all of its variants.
 mcfftResult create_batch(mcfftPlan* plan, const mcfftDesc* descs, int count,
-                         mcfftPrecision precision, unsigned flags, bool by_shape, bool* indexed) {
+                         mcfftPrecision precision, unsigned flags, bool by_shape, bool reg,
+                         bool* indexed) {
   mcfftPlan p = nullptr;
   mcfftResult r = plan_begin(plan, precision, flags, &p);
   if (r) return r;
@@ -1884,6 +2031,8 @@ mcfftResult create_batch(mcfftPlan* plan, const mcfftDesc* descs, int count,
     }
   }
   p->queue_planned = groups.size() > 1;
+  p->reg_queue = reg && p->queue_planned;
+  if (reg && !p->reg_queue) r = MCFFT_UNSUPPORTED_SIZE;
   if (const char* e = std::getenv("MCFFT_QUEUE")) p->queue_planned = std::atoi(e) != 0;
   for (size_t gi = 0; gi < groups.size() && !r; ++gi) {
     const Group& g = groups[gi];
@@ -1946,13 +2095,21 @@ mcfftResult mcfftPlanCreateBatch(mcfftPlan* plan, const mcfftDesc* descs, int co
   // instead (MCFFT_GROUPING=adjacent forces that).
   bool by_shape = true;
   if (const char* e = std::getenv("MCFFT_GROUPING")) by_shape = std::strcmp(e, "adjacent") != 0;
-  if (by_shape) {
+  // Plain plans first try the one-launch kernel on the register passes, then
+  // the batch kernel.
+  const bool reg = precision == MCFFT_PREC_FP16 && !std::getenv("MCFFT_QUEUE") &&
+                   !std::getenv("MCFFT_TILE_POINTS") && !std::getenv("MCFFT_NO_TILE");
+  for (int bs = by_shape ? 1 : 0; bs >= 0; --bs) {
     bool indexed = false;
-    const mcfftResult r = create_batch(plan, descs, count, precision, flags, true, &indexed);
-    if (r != MCFFT_UNSUPPORTED_SIZE || !indexed) return r;
+    mcfftResult r = MCFFT_UNSUPPORTED_SIZE;
+    if (reg) r = create_batch(plan, descs, count, precision, flags, bs != 0, true, &indexed);
+    if (r == MCFFT_UNSUPPORTED_SIZE) {
+      indexed = false;
+      r = create_batch(plan, descs, count, precision, flags, bs != 0, false, &indexed);
+    }
+    if (bs == 0 || r != MCFFT_UNSUPPORTED_SIZE || !indexed) return r;
   }
-  bool unused = false;
-  return create_batch(plan, descs, count, precision, flags, false, &unused);
+  return MCFFT_UNSUPPORTED_SIZE;
 }
 
 mcfftResult mcfftPlanCreate1d(mcfftPlan* plan, int64_t n, int64_t batch, mcfftPrecision precision,
@@ -2039,6 +2196,7 @@ mcfftResult mcfftPlanDestroy(mcfftPlan p) {
   if (p->capture_stream) cudaStreamDestroy(p->capture_stream);
   for (void* d : p->allocs) cudaFree(d);
   delete p->q.args;
+  delete p->q.rargs;
   delete p;
   return MCFFT_SUCCESS;
 }

@@ -48,6 +48,11 @@ void reg_stagings(const TileKernel& k, layout::Kind ik, layout::Kind ok, int in_
   *out = reg_staging_out(s, ik, ok, out_elem, out_sp, out_sc, out_so, ncols, nouter);
 }
 
+bool reg_gather_staging(const TileKernel& k, bool out, int elem, const std::vector<int64_t>& offs,
+                        layout::Staging* st, std::vector<int32_t>* tab) {
+  return reg_gather_staging(RegShape{k.L, k.R, k.C, k.reg_h, k.mma}, out, elem, offs, st, tab);
+}
+
 cudaError_t gen_reg_twiddles(void* dst, int L, int NV, int mode, int sign, double scale,
                              cudaStream_t st) {
   const int n = mode == 2 ? L / 2 : L, threads = 256;

@@ -23,6 +23,9 @@ void reg_stagings(const TileKernel& k, layout::Kind ik, layout::Kind ok, int in_
                   int64_t in_sp, int64_t in_sc, int64_t in_so, int64_t out_sp, int64_t out_sc,
                   int64_t out_so, int64_t ncols, int64_t nouter, layout::Staging* in,
                   layout::Staging* out);
+// The same for transforms at unrelated offsets (reg_staging.h).
+bool reg_gather_staging(const TileKernel& k, bool out, int elem, const std::vector<int64_t>& offs,
+                        layout::Staging* st, std::vector<int32_t>* tab);
 
 // Phase-1 twiddles W_L^(k v) * scale in the layout of RegPass (mode 0: FP32,
 // 8 bytes at k NV + v; 1: doubled for two columns, 16 bytes; 2: pairs (2i,
@@ -40,6 +43,7 @@ TileKernel make_reg() {
   k.reg_kind = KIND;
   k.reg_h = P::h;
   k.tw_bytes = P::TWB;
+  k.tab_bytes = P::TABB;
   k.tw_mode = P::PK ? (R1 == 32 ? 2 : 1) : 0;
   return k;
 }
@@ -53,6 +57,7 @@ TileKernel make_mma() {
   k.fn_inv = reinterpret_cast<const void*>(&reg::fft_reg<Q>);
   k.reg_kind = KIND;
   k.tw_bytes = P::TWB;
+  k.tab_bytes = P::TABB;
   k.mma = true;
   k.fill_tw[0] = &P::fill_twiddles;
   k.fill_tw[1] = &Q::fill_twiddles;
@@ -69,6 +74,7 @@ TileKernel make_mma_rows() {
   k.fn_inv = reinterpret_cast<const void*>(&reg::fft_reg<Q>);
   k.reg_kind = reg::kRR;
   k.tw_bytes = P::TWB;
+  k.tab_bytes = P::TABB;
   k.mma = true;
   k.fill_tw[0] = &P::fill_twiddles;
   k.fill_tw[1] = &Q::fill_twiddles;

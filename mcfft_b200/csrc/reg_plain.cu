@@ -34,6 +34,7 @@ const std::vector<TileKernel>& reg_registry_plain() {
       make_mma<512, reg::kRR, false, 4096>(),
       make_mma<1024, reg::kRR, false, 4096>(),
       make_mma_rows<reg::Mma4096<false>, reg::Mma4096<true>>(),
+      make_mma_rows<reg::Mma4096<false, 16384>, reg::Mma4096<true, 16384>>(),
       make_mma_rows<reg::Mma2048<false>, reg::Mma2048<true>>()};
   return v;
 }

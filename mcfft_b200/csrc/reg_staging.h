@@ -2,6 +2,8 @@
 // and where it takes the result from: tensor-map dimensions of the layouts
 // that RegPass (fft_reg.cuh) and MmaPass (fft_mma.cuh) address.
 #pragma once
+#include <vector>
+
 #include "layout.h"
 
 namespace mcfft {
@@ -96,6 +98,40 @@ inline layout::Staging reg_rows_staging(const RegShape& k, bool out, int elem, i
   reg_add_dim(&s, ncols, k.C, sc, k.C, 0);
   if (nouter > 1) reg_add_dim(&s, nouter, 1, so, 0, 1);
   return s;
+}
+
+// Transforms at unrelated offsets, each copied by itself: box = one
+// transform of the row layouts that keep a column's rows together; `tab`
+// receives each transform's first 32-point row.  False if the variant's
+// layout or an offset does not allow it.
+inline bool reg_gather_staging(const RegShape& k, bool out, int elem, const std::vector<int64_t>& offs,
+                               layout::Staging* st, std::vector<int32_t>* tab) {
+  if (!k.mma || k.L < 256 || elem != 4) return false;
+  // positions split as [rows of a box's last dimension][dim 1]: see
+  // reg_row_staging, reg_rows_staging
+  const bool inner = k.L > 1024 && !(out && k.L == 2048);
+  const int rows = inner ? k.L / 512 : k.L / 32, step = 32 * (k.L / 512);
+  int64_t last = 0;
+  tab->clear();
+  for (int64_t o : offs) {
+    if (o < 0 || o % 32 || (o + k.L) / 32 >= (int64_t(1) << 31)) return false;
+    tab->push_back((int32_t)(o / 32));
+    last = o > last ? o : last;
+  }
+  layout::Staging s;
+  s.kind = layout::ROW;
+  s.L = k.L;
+  s.C = k.C;
+  s.elem = elem;
+  s.E = 32;
+  s.row_bytes = 128;
+  s.swz = 7;
+  reg_add_dim(&s, 32, 32, 1, 0, 0);
+  if (inner) reg_add_dim(&s, 16, 16, step, 0, 0);
+  else reg_add_dim(&s, 1, 1, 32, 0, 0);
+  reg_add_dim(&s, last / 32 + rows, rows, 32, 0, 0);
+  *st = s;
+  return true;
 }
 
 inline layout::Staging reg_staging_in(const RegShape& k, layout::Kind ik, int elem, int64_t sp, int64_t sc,

@@ -467,6 +467,37 @@ static void check_mma2048() {
   printf("%s 2048-point rows, plain\n", g_bad == bad0 ? "ok" : "FAULT");
 }
 
+// Transforms copied one by one land where a tile's own box would put them.
+static void check_gather(int L, int R) {
+  const int bad0 = g_bad, C = 16384 / L;
+  const RegShape sh{L, R, C, 0, true};
+  const std::vector<int64_t> offs{0, 3 * int64_t(L), L + 32};
+  for (int out = 0; out < 2; ++out) {
+    const auto want = tma_place(out ? reg_staging_out(sh, layout::ROW, layout::ROW, 4, 1, L, 0, C, 1)
+                                    : reg_staging_in(sh, layout::ROW, 4, 1, L, 0, C, 1), true);
+    layout::Staging g;
+    std::vector<int32_t> tab;
+    CHECK(reg_gather_staging(sh, out, 4, offs, &g, &tab) && tab.size() == offs.size() && g.ndims == 3, "no map");
+    CHECK((int)(g.box[0] * g.box[1] * g.box[2]) == L, "box");
+    for (size_t t = 0; t < offs.size(); ++t) {
+      CHECK((uint64_t)tab[t] + g.box[2] <= g.gdim[2], "row %d outside the map", tab[t]);
+      for (int c = 0; c < C; ++c)  // column c at byte c L 4 of the buffer
+        for (int i = 0; i < L; ++i) {
+          const int64_t x = i % g.box[0], y = i / g.box[0] % g.box[1], z = i / (g.box[0] * g.box[1]);
+          const int64_t e = x + y * (int64_t)g.gstride_bytes[1] / 4 + (tab[t] + z) * (int64_t)g.gstride_bytes[2] / 4;
+          uint32_t off = (uint32_t)(c * L + i) * 4;
+          off ^= ((off >> 7) & g.swz) << 4;
+          const int64_t pos = e - offs[t];
+          CHECK(pos >= 0 && pos < L && want[pos * C + c] == off, "point %lld", (long long)pos);
+        }
+    }
+  }
+  layout::Staging g;
+  std::vector<int32_t> tab;
+  CHECK(!reg_gather_staging(sh, false, 4, {16}, &g, &tab), "offset of half a row");
+  printf("%s %d-point gathered rows\n", g_bad == bad0 ? "ok" : "FAULT", L);
+}
+
 // 4096-point rows, FP32 exchange.
 static void check_reg4096() {
   using M = Reg4096<false, false>;
@@ -520,6 +551,7 @@ static void check_reg4096() {
 int main() {
   check_mma4096();
   check_mma2048();
+  check_gather(256, 1), check_gather(512, 2), check_gather(1024, 4), check_gather(2048, 8), check_gather(4096, 16);
   check_reg4096();
   W(256, kRR, false), W(512, kRR, false), W(1024, kRR, false);
   WS(256), WS(512), WS(1024);

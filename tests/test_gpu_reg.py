@@ -91,3 +91,56 @@ def test_columns(shape, batch, form):
                                          ((2048, 128), 5)])
 def test_rows_2048(shape, batch, direction):
     _check(shape, batch, "plain", direction)
+
+
+# every variant of the one-launch kernel: 1D lengths of one pass and of two,
+# 2D and 3D shapes; counts that leave ragged tiles
+UNEVEN = [((64,), 1), ((128,), 300), ((256,), 67), ((512,), 33), ((1024,), 17), ((2048,), 9), ((4096,), 5),
+          ((1 << 13,), 3), ((1 << 14,), 3), ((1 << 15,), 2), ((1 << 17,), 2), ((1 << 18,), 1), ((1 << 20,), 1),
+          ((1 << 19,), 1), ((64, 2048), 3), ((64, 64), 3), ((128, 1024), 2), ((512, 256), 2), ((1024, 512), 1), ((64, 64, 128), 1)]
+
+
+def _uneven(shapes, order, direction, execs=3):
+    """One descriptor per transform; inputs packed in the given order, outputs
+    in the opposite one.  Returns the results transform by transform."""
+    items = [s for s, c in shapes for _ in range(c)]
+    rng = np.random.default_rng(11)
+    if order == "mixed":
+        rng.shuffle(items)
+    size = [int(np.prod(s)) for s in items]
+    io = np.concatenate([[0], np.cumsum(size)])
+    oo = [int(io[-1] - e) for e in io[1:]] if order == "mixed" else io[:-1]
+    descs = [(s, 1, int(a), int(b)) for s, a, b in zip(items, io, oo)]
+    total = int(io[-1])
+    x = rng.uniform(-1, 1, total) + 1j * rng.uniform(-1, 1, total)
+    xd = to_device(x, True)
+    out = torch.empty(total, dtype=torch.complex32, device="cuda")
+    with mc.Plan(descs=descs, precision=mc.PREC_FP16) as p:
+        if order == "packed" or min(size) >= 256:
+            assert p.info().launches == 1
+        for _ in range(execs):  # the counters of one exec are the next one's
+            out.view(torch.uint8).fill_(0xFF)
+            p.exec_ptr(xd.data_ptr(), out.data_ptr(), direction, torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        p.check_status()
+    return descs, rounded(x, True), from_device(out)
+
+
+@pytest.mark.parametrize("direction", [mc.FORWARD, mc.INVERSE])
+@pytest.mark.parametrize("order", ["packed", "mixed"])
+@pytest.mark.parametrize("shapes", [UNEVEN, [s for s in UNEVEN if s[0] not in ((64,), (128,), (64, 64))],
+                                    [((256,), 65), ((512,), 1)]])
+def test_uneven_one_launch(shapes, order, direction):
+    """Against the oracle: the packed batch, transforms at unrelated offsets
+    (with 64 or 128 points among them: other kernels), and a batch whose
+    tables all stay in shared memory."""
+    descs, xr, y = _uneven(shapes, order, direction)
+    worst = 0.0
+    for shape, _, io, oo in descs:
+        n = int(np.prod(shape))
+        v = xr[io:io + n].reshape((1,) + tuple(shape))
+        ref = oracle.fftnd(v, list(shape)) if direction == mc.FORWARD else \
+            np.conj(oracle.fftnd(np.conj(v), list(shape)))
+        rel, _ = compare(y[oo:oo + n], ref / n)
+        worst = max(worst, rel)
+    assert worst < 1e-3, worst
