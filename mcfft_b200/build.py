@@ -28,7 +28,7 @@ SOURCES = ["tables.cu", "pass_kernels.cu", "tile_pass.cu", "tile_split.cu", "que
            "reg_pass.cu", "reg_plain.cu", "reg_split.cu", "reg_split16.cu",
            "reg_queue.cu", "reg_queue_plain_fwd.cu", "reg_queue_plain_inv.cu", "layout.cpp", "mcfft_api.cu", "noalloc.cu", "norms.cu"]
 HEADERS = ["sm100_ptx.cuh", "tail_layout.h", "fft_pass.cuh", "fft_pass_split.cuh", "fft_tile.cuh",
-           "fft_tile_split.cuh", "fft_codelets.cuh", "fft_reg.cuh", "fft_mma.cuh", "fft_rows.cuh", "reg_pass.h",
+           "fft_tile_split.cuh", "fft_codelets.cuh", "fft_reg.cuh", "fft_mma.cuh", "fft_rows.cuh", "fft_small.cuh", "reg_pass.h",
            "reg_staging.h", "reg_queue.cuh", "reg_queue.h", "fft_queue.cuh", "queue.h", "queue_order.h", "host_schedule.h",
            "tile_pass.h", "layout.h", "mcfft_internal.h"]
 

@@ -85,7 +85,7 @@ struct MmaPass {
   static constexpr int T = TP / 32, NW = T / 32, NG = 1;
   static constexpr bool BIG = T == 512;
   static constexpr int NBUF = BIG ? 3 : 2, NFULL = NBUF, THREADS = T + (BIG ? 128 : 32), MINB = BIG ? 1 : 3;
-  static constexpr int BUF = TP * 4;
+  static constexpr int BUF = TP * 4, EI = 4, EO = 4;
   static constexpr bool ROWIN = KIND != kCC;
   // Phase 2 of row-input passes of 256 and 512 points reads the four operand
   // slots of a vector as one chunk (WK); elsewhere a chunk is four vectors.
@@ -180,6 +180,11 @@ struct MmaPass {
                        : KNC{warp, 0, g0 | u0 << 1 | u1 << 2 | g1 << 3 | g2 << 4 | u2 << 5};
   }
   static __host__ __device__ constexpr u32 v_of(u32 n2, u32 n3) { return n2 * R + n3; }
+
+  // Row kinds: byte in the tile's transforms, one after another, of byte off
+  // of the buffer.
+  static __host__ __device__ constexpr u32 in_map(u32 off) { return off ^ ((off >> 3) & 0x70u); }
+  static __host__ __device__ constexpr u32 out_map(u32 off) { return in_map(off); }
 
   // Offsets of a thread's chunks: thread part, and register part (linear).
   static constexpr u32 XM = 0x70u;

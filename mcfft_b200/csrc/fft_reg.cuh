@@ -306,6 +306,15 @@ struct RegPass {
     return make_float2(cs, INV ? sn : -sn);
   }
 
+  // Row kind: byte in the tile's transforms, one after another, of byte off of
+  // the buffer (swizzled 128-byte rows, the columns' side by side).
+  template <int E>
+  static __host__ __device__ constexpr uint32_t row_map(uint32_t off) {
+    return ((off >> 7) % C) * (L * E) + (off >> 7) / C * 128u + ((off ^ off >> 3) & 0x70u) + (off & 15u);
+  }
+  static __host__ __device__ constexpr uint32_t in_map(uint32_t off) { return row_map<EI>(off); }
+  static __host__ __device__ constexpr uint32_t out_map(uint32_t off) { return row_map<EO>(off); }
+
   // Tables that depend on the plan (none here).
   template <class A>
   static __device__ __forceinline__ void setup(const A&, uint8_t*, int) {}

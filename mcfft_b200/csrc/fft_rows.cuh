@@ -63,6 +63,11 @@ struct Mma4096 {
   static __host__ __device__ constexpr u32 out_at(u32 k1, u32 k2, u32 k3) {
     return ((k2 >> 1) * 16 + k3) * 128 + ((((k2 & 1u) << 2 | k1 >> 2) ^ (k3 & 7u)) << 4) + (k1 & 3u) * 4;
   }
+  // byte in the transforms, one after another, of byte off of the buffer
+  static __host__ __device__ constexpr u32 in_map(u32 off) {
+    return (off & ~0x3fffu) + ((off >> 7) & 15u) * 1024 + ((off >> 11) & 7u) * 128 + ((off ^ off >> 3) & 0x70u) + (off & 15u);
+  }
+  static __host__ __device__ constexpr u32 out_map(u32 off) { return in_map(off); }
   // ------------------------------------------------- who handles which point
   struct XY {
     u32 x, y;
@@ -277,6 +282,8 @@ struct Reg4096 {
   // k1; phase 3: x = k1, y = k2.
   static __host__ __device__ constexpr u32 xd(u32 t) { return t & 15u; }
   static __host__ __device__ constexpr u32 yd(u32 t, u32 j) { return ((t >> 4) & 1u) | j << 1 | (t >> 5) << 2; }
+  static __host__ __device__ constexpr u32 in_map(u32 off) { return off; }
+  static __host__ __device__ constexpr u32 out_map(u32 off) { return off; }
   // Slot of phase 2's output: 16-byte chunks of row (k1, k2) XORed with k1.
   static __host__ __device__ constexpr u32 ex2_at(u32 k1, u32 k2, u32 n3) {
     return (k1 * 256 + k2 * 16 + (n3 ^ ((k1 & 7u) << 1))) * 8;
@@ -301,6 +308,12 @@ struct Reg4096 {
   template <class A>
   static __device__ __forceinline__ void run(const A&, const State&, u32 sb, u32 tws, int t, u32,
                                              const Sync<T>&) {
+    phases<false>(sb, tws, t, nullptr, nullptr);
+  }
+  // G: the transform read from and written to global memory (every access of
+  // a half warp is a line), the tables complete after the wait.
+  template <bool G>
+  static __device__ __forceinline__ void phases(u32 sb, u32 tws, int t, const uint8_t* gin, uint8_t* gout) {
     const u32 x = xd(t);
     {
       float re[2][16], im[2][16];
@@ -310,13 +323,17 @@ struct Reg4096 {
 #pragma unroll
         for (int n = 0; n < 16; ++n) {
           float2 z;
-          if constexpr (IN16_) z = sm100::unpack_half2(lds32(b + n * 256 * EI));
+          if constexpr (G && IN16_)
+            z = sm100::unpack_half2(*reinterpret_cast<const u32*>(gin + (yd(t, j) * 16 + x) * 4 + n * 1024));
+          else if constexpr (G) z = *reinterpret_cast<const float2*>(gin + (yd(t, j) * 16 + x) * 8 + n * 2048);
+          else if constexpr (IN16_) z = sm100::unpack_half2(lds32(b + n * 256 * EI));
           else z = lds64f(b + n * 256 * EI);
           re[j][n] = z.x;
           im[j][n] = z.y;
         }
       }
-      if constexpr (EI != EO) col_bar<128>(4);
+      if constexpr (G) asm volatile("cp.async.wait_all;" ::: "memory");
+      if constexpr (G || EI != EO) col_bar<128>(4);
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
         const u32 y = yd(t, j), b = sb + (y * 16 + x) * 8;
@@ -374,13 +391,17 @@ struct Reg4096 {
           im[j][2 * n + 1] = z.w;
         }
       }
-      col_bar<128>(4);
+      if constexpr (!G) col_bar<128>(4);
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
-        const u32 b = sb + (yd(t, j) * 16 + x) * 8;
+        const u32 o = (yd(t, j) * 16 + x) * 8;
         Dft<16, INV, float>::run(re[j], im[j]);
 #pragma unroll
-        for (int k = 0; k < 16; ++k) tile::sts64(b + k * 256 * 8, make_float2(re[j][k], im[j][k]));
+        for (int k = 0; k < 16; ++k) {
+          const float2 z = make_float2(re[j][k], im[j][k]);
+          if constexpr (G) *reinterpret_cast<float2*>(gout + o + k * 256 * 8) = z;
+          else tile::sts64(sb + o + k * 256 * 8, z);
+        }
       }
     }
   }

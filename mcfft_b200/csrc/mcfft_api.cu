@@ -387,7 +387,7 @@ bool gather_rows(const layout::Staging& tile_st, int64_t L, int64_t C,
 
 // Row passes of few points take 4096-point tiles (four warps, three CTAs per
 // SM), which spread over the SMs and have a quarter of the latency.  Measured
-// on a B200, back-to-back execs, 4096-point against full tiles: 1024 x 8 6.2
+// on a B200 with TMA, back-to-back execs, 4096-point against full tiles: 1024 x 8 6.2
 // against 8.2 us, 256 x 1000 4.1 / 7.5, 64 x 5000 4.1 / 8.2, 512 x 5000 8.2 /
 // 10.3, 512 x 9001 14.3 / 14.3.  Past about four full tiles per SM the two
 // tie, and as the first pass of a 2D transform the full tiles are faster
@@ -396,6 +396,15 @@ bool small_tiles(const mcfftPlan p, const PassSpec& s) {
   if (s.L == 4096) return true;  // the register kernel of this length has one tile size
   return s.in_sp == 1 && s.out_sp == 1 && s.L * s.ncols * s.nouter <= int64_t(4) * p->sms * 16384;
 }
+
+// The most 4096-point tiles of contiguous rows that run without TMA
+// (fft_small.cuh), one CTA each.  Measured on a B200, back-to-back execs, with
+// TMA against without: plain 1024 x 8 6.15 / 4.10 us, 4096 x 256 8.2 / 6.15,
+// 512 x 9001 14.3 / 12.3, 4096 x 2300 25.7 / 24.6, 4096 x 4000 36.8 / 38.9;
+// FP32 exchange 4096 x 256 8.2 / 6.3, x 592 14.5 / 12.3, x 1024 18.7 / 20.5,
+// 512 x 9001 16.6 / 16.6, 64 x 100000 (FP16 in) 16.9 / 18.1: past a few tiles
+// per CTA slot the copying warps' run-ahead is worth more than the short start.
+int64_t direct_tiles(const mcfftPlan p) { return int64_t(p->split ? 6 : 16) * p->sms; }
 
 // Builds a pass on the TMA-fed kernel.  Returns MCFFT_UNSUPPORTED_SIZE when
 // the shape is outside what that kernel handles (the caller falls back).
@@ -587,6 +596,12 @@ mcfftResult add_tile_pass(mcfftPlan p, const PassSpec& s, int only_tile_points =
   }
   occ = std::max(1, k->tmem_cols ? std::min(occ, 512 / k->tmem_cols) : occ);
   tp.grid = (int)std::min<int64_t>(a.ntiles, (int64_t)p->sms * occ);
+  if (k->fn_small[0] && !indexed && s.nouter == 1 && s.in_sc == s.L && s.out_sc == s.L &&
+      a.ntiles <= direct_tiles(p)) {
+    tp.small = true;
+    tp.small_points = s.ncols * s.L;
+    tp.grid = (int)a.ntiles;
+  }
   ps.in_buf = s.in_buf; ps.out_buf = s.out_buf;
   ps.in_f16 = s.in_f16; ps.out_f16 = s.out_f16;
   ps.in_off = s.in_off; ps.out_off = s.out_off;

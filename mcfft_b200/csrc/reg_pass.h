@@ -4,6 +4,7 @@
 #include "fft_mma.cuh"
 #include "fft_reg.cuh"
 #include "fft_rows.cuh"
+#include "fft_small.cuh"
 #include "tile_pass.h"
 
 namespace mcfft {
@@ -33,6 +34,17 @@ bool reg_gather_staging(const TileKernel& k, bool out, int elem, const std::vect
 cudaError_t gen_reg_twiddles(void* dst, int L, int NV, int mode, int sign, double scale,
                              cudaStream_t st);
 
+// The kernels without TMA of a 4096-point row tile.
+template <class P, class Q>
+void add_small(TileKernel* k) {
+  if constexpr (P::TP == 4096 && P::KIND == reg::kRR) {
+    k->fn_small[0] = reinterpret_cast<const void*>(&reg::fft_small<P>);
+    k->fn_small[1] = reinterpret_cast<const void*>(&reg::fft_small<Q>);
+    k->small_smem = reg::small_smem<P>();
+    k->small_threads = P::T;
+  }
+}
+
 template <int L, int R1, int R2, int TP, bool IN16, bool OUT16, int KIND, bool POST>
 TileKernel make_reg() {
   using P = reg::RegPass<L, R1, R2, TP, IN16, OUT16, KIND, POST, false>;
@@ -45,6 +57,7 @@ TileKernel make_reg() {
   k.tw_bytes = P::TWB;
   k.tab_bytes = P::TABB;
   k.tw_mode = P::PK ? (R1 == 32 ? 2 : 1) : 0;
+  add_small<P, Q>(&k);
   return k;
 }
 
@@ -63,6 +76,7 @@ TileKernel make_mma() {
   k.fill_tw[1] = &Q::fill_twiddles;
   k.fill_frag[0] = &P::fill_fragments;
   k.fill_frag[1] = &Q::fill_fragments;
+  add_small<P, Q>(&k);
   return k;
 }
 
@@ -80,6 +94,7 @@ TileKernel make_mma_rows() {
   k.fill_tw[1] = &Q::fill_twiddles;
   k.fill_frag[0] = &P::fill_fragments;
   k.fill_frag[1] = &Q::fill_fragments;
+  add_small<P, Q>(&k);
   return k;
 }
 // 4096-point rows, FP32 exchange.
@@ -94,6 +109,7 @@ TileKernel make_reg4096() {
   k.tw_bytes = P::TWB;
   k.fill_tw[0] = &P::fill_twiddles;
   k.fill_tw[1] = &Q::fill_twiddles;
+  add_small<P, Q>(&k);
   return k;
 }
 

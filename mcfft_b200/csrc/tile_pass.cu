@@ -12,6 +12,7 @@
 
 #include "fft_tile.cuh"
 #include "layout.h"
+#include "fft_small.cuh"
 #include "tile_pass.h"
 
 namespace mcfft {
@@ -167,6 +168,23 @@ bool tile_check_encode(const layout::Staging& s, const void* probe) {
 
 cudaError_t launch_tile_pass(const TilePass& tp, const void* in, void* out, int dir,
                              cudaStream_t st, bool pdl) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  cfg.gridDim = dim3(tp.grid);
+  cfg.stream = st;
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl ? 1 : 0;
+  if (tp.small) {
+    if (!in || !out || (reinterpret_cast<uintptr_t>(in) & 15) || (reinterpret_cast<uintptr_t>(out) & 15))
+      return cudaErrorInvalidValue;  // as an encoding of the tensor maps
+    SmallArgs s{in, out, tp.tw[dir], tp.bmat[dir], (uint64_t)tp.small_points};
+    cfg.blockDim = dim3(tp.k->small_threads);
+    cfg.dynamicSmemBytes = (size_t)tp.k->small_smem;
+    void* args[] = {&s};
+    return cudaLaunchKernelExC(&cfg, tp.k->fn_small[dir ? 1 : 0], args);
+  }
   TileArgs a = tp.args;
   if (!encode(&a.tmap_in, tp.lay.in, in) || !encode(&a.tmap_out, tp.lay.out, out))
     return cudaErrorInvalidValue;
@@ -195,16 +213,8 @@ cudaError_t launch_tile_pass(const TilePass& tp, const void* in, void* out, int 
     }
   }
   void* args[] = {&a};
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(tp.grid);
   cfg.blockDim = dim3(tp.k->nthreads);
   cfg.dynamicSmemBytes = (size_t)tp.k->smem_bytes;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = pdl ? 1 : 0;
   return cudaLaunchKernelExC(&cfg, fn, args);
 }
 

@@ -33,6 +33,9 @@ struct TileKernel {
   bool mma = false;
   void (*fill_tw[2])(float*) = {nullptr, nullptr};
   void (*fill_frag[2])(uint32_t*) = {nullptr, nullptr};
+  // 4096-point row tiles: the kernels without TMA (fft_small.cuh).
+  const void* fn_small[2] = {nullptr, nullptr};
+  int small_smem = 0, small_threads = 0;
   const void* fn_of(int dir) const { return dir && fn_inv ? fn_inv : fn; }
 };
 
@@ -45,6 +48,8 @@ struct TilePass {
   layout::PassLayout lay;
   TileArgs args{};  // everything except tensor maps and per-direction tables
   int grid = 1;
+  bool small = false;  // run by k->fn_small: small_points points in all
+  int64_t small_points = 0;
   const float4* tw[2] = {nullptr, nullptr};
   const float2* tail[2] = {nullptr, nullptr};
   const float2* post_a[2] = {nullptr, nullptr};

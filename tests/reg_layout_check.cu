@@ -74,6 +74,24 @@ static std::vector<uint32_t> tma_place(const layout::Staging& s, bool row) {
   return at;
 }
 
+// The kernels without TMA copy 16 bytes of a transform to where TMA would
+// (in_map, out_map: the inverse of the tensor map's placement).
+template <class P>
+void check_maps(const RegShape& sh, const char* name) {
+  const int bad0 = g_bad;
+  for (int out = 0; out < 2; ++out) {
+    const uint32_t e = out ? P::EO : P::EI;
+    const auto at = tma_place(out ? reg_staging_out(sh, layout::ROW, layout::ROW, e, 1, P::L, 0, P::C, 1)
+                                  : reg_staging_in(sh, layout::ROW, e, 1, P::L, 0, P::C, 1), true);
+    for (uint32_t c = 0; c < P::C; ++c)
+      for (uint32_t p = 0; p < P::L; ++p) {
+        const uint32_t x = at[p * P::C + c], a = x & ~15u;
+        CHECK((out ? P::out_map(a) : P::in_map(a)) + (x & 15u) == (c * P::L + p) * e, "byte %u", x);
+      }
+  }
+  printf("%s %s maps\n", g_bad == bad0 ? "ok" : "FAULT", name);
+}
+
 template <class P>
 void check(const char* name) {
   const int bad0 = g_bad;
@@ -553,6 +571,15 @@ int main() {
   check_mma2048();
   check_gather(256, 1), check_gather(512, 2), check_gather(1024, 4), check_gather(2048, 8), check_gather(4096, 16);
   check_reg4096();
+#define MM(L) check_maps<MmaPass<L, kRR, false, false, 4096>>({L, L / 256, 4096 / L, 0, true}, #L)
+  MM(256), MM(512), MM(1024);
+  check_maps<Mma4096<false>>({4096, 16, 1, 0, true}, "4096");
+  check_maps<Reg4096<true, false>>({4096, 16, 1, 0, false}, "4096 FP16 in");
+  check_maps<Reg4096<false, false>>({4096, 16, 1, 0, false}, "4096 FP32");
+#define RM(L, R1, I, O) check_maps<RegPass<L, R1, L / R1, 4096, I, O, kRR, false, false>>({L, R1, 4096 / L, 0, false}, #L " " #I " " #O)
+  RM(64, 8, true, true), RM(128, 8, true, true);
+  RM(64, 8, true, false), RM(128, 8, true, false), RM(256, 16, true, false), RM(512, 16, true, false);
+  RM(64, 8, false, false), RM(128, 8, false, false), RM(256, 16, false, false), RM(512, 16, false, false);
   W(256, kRR, false), W(512, kRR, false), W(1024, kRR, false);
   WS(256), WS(512), WS(1024);
   W(256, kRC, false), W(512, kRC, false), W(1024, kRC, false);
