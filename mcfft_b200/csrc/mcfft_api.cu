@@ -1559,10 +1559,12 @@ mcfftResult build_queue(mcfftPlan p) {
 
 // The queue of a plan for the one-launch kernel on the register passes
 // (reg_queue.cuh), in the same order.  MCFFT_UNSUPPORTED_SIZE: the caller
-// plans for the batch kernel instead.  Chunks of 16 first-pass tiles per CTA:
-// a batch of 4096 1D transforms of 2^8 .. 2^16 points and 64 of 128 .. 512
-// points a side takes 241 us (14 runs of one pass per CTA), in chunks of 8
-// 242 .. 246, of 4 249, of 32 240; the batch kernel takes 350 us.
+// plans for the batch kernel instead.  Chunks of 8 first-pass tiles per CTA,
+// a key's readers at least 6 tiles per CTA behind it: a batch of 4096 1D
+// transforms of 2^8 .. 2^16 points and 64 of 128 .. 512 points a side takes
+// 235 us (chunks of 16: 242, of 6: 238), one of 1600 such 2D transforms 405
+// (423, 391), one of 16000 and 250 805 (797, 798).  The batch kernel takes 350
+// us for the first.
 mcfftResult build_reg_queue(mcfftPlan p) {
   const size_t np = p->passes.size();
   if (np > (size_t)kRegQueueMaxPasses || p->no_queue) return MCFFT_UNSUPPORTED_SIZE;
@@ -1577,7 +1579,7 @@ mcfftResult build_reg_queue(mcfftPlan p) {
   if (G <= 0) return MCFFT_UNSUPPORTED_SIZE;
   Queue& q = p->q;
   q.resident = tabs <= reg::QueueShape::TAB_BYTES;
-  int64_t QC = 16, lag = 0;
+  int64_t QC = 8, lag = 6;
   if (const char* e = std::getenv("MCFFT_QUEUE_CHUNK")) QC = std::max<int64_t>(1, std::atoll(e));
   if (const char* e = std::getenv("MCFFT_QUEUE_LAG")) lag = std::max<int64_t>(0, std::atoll(e));
   const std::vector<QOrderItem> order = queue_order(queue_passes(p), G, QC, lag);

@@ -64,6 +64,8 @@ bool fill_rpass(const TilePass& tp, int dir, const void* in, void* out, RPass* q
   q->col_blocks = (uint32_t)a.col_blocks;
   q->in_tile_bytes = a.in_tile_bytes;
   q->variant = reg_queue_variant(*tp.k);
+  q->tw_bytes = (uint32_t)tp.k->tw_bytes;
+  q->tab_bytes = (uint32_t)tp.k->tab_bytes;
   q->wait_base = q->sig_base = -1;
   q->sig_mul = q->sig_div = 1;
   return q->variant >= 0;

@@ -3,11 +3,10 @@
 // Mma4096).
 //
 // What bounds it: in a long run of one pass HBM, as in the pass kernels
-// (2^16 x 1024 in 194 us, 190 as two launches); in a batch of many shapes also
-// the switches from pass to pass, each of which waits for its tables.
-// Measured, uneven batches of 1D lengths 2^8 .. 2^16 and some 2D shapes, batch
-// kernel (fft_queue.cuh) against this one: 4160 transforms 349 / 248 us, 1015
-// 116 / 78, 304 48 / 20, 65 37 / 20.
+// (2^16 x 1024 in 194 us, 190 as two launches).  Measured, uneven batches of
+// 1D lengths 2^8 .. 2^16 and some 2D shapes, batch kernel (fft_queue.cuh)
+// against this one: 4160 transforms 349 / 235 us, 1015 116 / 78, 304 48 / 19,
+// 65 37 / 19 (tables loaded only at the start of a run: 243, 80, 21, 21).
 //
 // The queue is the batch kernel's (queue_order.h): items of (pass, tile),
 // dealt to the CTAs in turn, every dependency pointing backwards, counters in
@@ -24,7 +23,8 @@
 // Why a switch over whole runs: the items of a CTA come in runs of one pass
 // (queue_order.h), and a routine's per-thread offsets and table are set up
 // once per run.  Tables stay in shared memory for the whole launch when those
-// of all passes fit (34 KB), else they are loaded at the start of a run.
+// of all passes fit (34 KB), else a run's table is copied while the last item
+// of the run before is worked on.
 //
 // The counters are zeroed by the last CTA to leave, for the next launch.
 // Every wait is bounded; a timeout sets the abort flag, after which all waits
@@ -33,6 +33,7 @@
 #include "fft_mma.cuh"
 #include "fft_reg.cuh"
 #include "fft_rows.cuh"
+#include "fft_small.cuh"
 
 namespace mcfft {
 
@@ -54,6 +55,7 @@ struct alignas(64) RPass {
   uint32_t in_tile_bytes;
   int32_t variant;
   uint32_t tw_off;  // resident tables: offset in the table area
+  uint32_t tw_bytes, tab_bytes;
   // Before loading tile (cb, outer): counters[wait_base + outer]
   // >= wait_count; wait_base -1: none.
   int32_t wait_base, wait_count;
@@ -250,32 +252,63 @@ __device__ __forceinline__ void queue_storer(const RArgs& a, const QueueBars& q,
   tile::tma_store_wait_all();
 }
 
-// Runs items k, k + 1, .. as long as they are of pass pi (tile routine X);
-// returns the first that is not.
+// A consumer thread's place in the queue.  Which pass an item is of is read
+// from the item list itself, two items ahead: also after a timeout every
+// thread runs the same items and meets the same barriers.
+struct QueuePlace {
+  const RItem* items;
+  uint32_t k = 0, nlocal, step;
+  RItem it, nx;
+  __device__ __forceinline__ QueuePlace(const RArgs& a, uint32_t n)
+      : items(a.items + blockIdx.x), nlocal(n), step(gridDim.x) {
+    it = nx = RItem{0u, 0u};
+    if (n) it = items[0];
+    nx = n > 1 ? items[step] : it;
+  }
+};
+
+// The table of the run at hand: runs alternate between the two ends of the
+// table area, so that a table can be copied while the one before is in use.
+struct TabState {
+  uint32_t off = 0, size = 0, end = 0;
+  __device__ __forceinline__ uint32_t next_off(const RPass& P) const {
+    return end ? 0u : ((uint32_t)QueueShape::TAB_BYTES - P.tab_bytes) & ~127u;
+  }
+  __device__ __forceinline__ bool fits(const RPass& P) const {
+    return size + P.tab_bytes + 128u <= (uint32_t)QueueShape::TAB_BYTES;
+  }
+  __device__ __forceinline__ static void copy(const RPass& P, uint32_t to, int t) {
+    for (uint32_t i = t; i < P.tw_bytes / 16; i += 512) cp_async16(to + 16 * i, P.tw + i, true);
+  }
+};
+
+// Runs the items from pl.k on as long as they are of one pass (tile routine
+// X); during the last of them the next run's table is on its way.
 template <class X>
-__device__ __forceinline__ uint32_t queue_run(const RPass& P, int pi, const MmaFrags& fr, const QueueBars& q,
-                                              uint32_t tab, int t, uint32_t k, uint32_t nlocal,
-                                              const Sync<512>& sync) {
+__device__ __forceinline__ void queue_run(const RArgs& a, const RPass& P, const MmaFrags& fr, const QueueBars& q,
+                                          uint32_t tab, const TabState& ts, int t, QueuePlace& pl,
+                                          const Sync<512>& sync) {
   constexpr uint32_t NBUF = QueueShape::NBUF;
   const uint32_t ncb = P.col_blocks;
   const RunState<X> st(P, fr, t);
   for (;;) {
-    const uint32_t b = k % NBUF;
-    X::run(P, st.get(fr), q.base_u + b * QueueShape::BUF, tab, t, q.ring[2 * b + 1] % ncb, sync);
+    const uint32_t k = pl.k, b = k % NBUF;
+    const RItem nn = k + 2 < pl.nlocal ? pl.items[(k + 2) * pl.step] : pl.nx;
+    const bool last = k + 1 >= pl.nlocal || pl.nx.pass != pl.it.pass;
+    if (last && !a.resident && k + 1 < pl.nlocal) {
+      const RPass& N = a.pass[pl.nx.pass];
+      if (ts.fits(N)) TabState::copy(N, q.base_u + QueueShape::OFF_TAB + ts.next_off(N), t);
+    }
+    wait_or_abort(&q.full[b], (k / NBUF) & 1u, q.abort_flag);
+    X::run(P, st.get(fr), q.base_u + b * QueueShape::BUF, tab, t, pl.it.tile % ncb, sync);
     sm100::fence_proxy_async_smem();
     __syncwarp();
     if ((t & 31) == 0) tile::mbar_arrive(&q.done[k % QueueShape::NDONE]);
-    if (++k >= nlocal) return k;
-    wait_or_abort(&q.full[k % NBUF], (k / NBUF) & 1u, q.abort_flag);
-    if ((int)q.ring[2 * (k % NBUF)] != pi) return k;
+    pl.it = pl.nx;
+    pl.nx = nn;
+    ++pl.k;
+    if (last) return;
   }
-}
-
-// A pass's tables into shared memory at `to`.
-template <class X>
-__device__ __forceinline__ void queue_tables(const RPass& P, uint8_t* to, int t) {
-  for (int i = t; i < X::TWB / 16; i += 512) *reinterpret_cast<float4*>(to + 16 * i) = __ldg(P.tw + i);
-  X::setup(P, to, t);
 }
 
 template <bool INV>
@@ -297,25 +330,30 @@ __global__ void __launch_bounds__(640, 1) fft_reg_queue(const __grid_constant__ 
     for (int f = 0; f < NBUF; ++f) sm100::mbar_init(&q.full[f], 1);
     for (int d = 0; d < QueueShape::NDONE; ++d) sm100::mbar_init(&q.done[d], NW);
     for (int b = 0; b < NBUF; ++b) sm100::mbar_init(&q.freeb[b], 1);
-    for (int i = 0; i < 2 * NBUF; ++i) q.ring[i] = 0;  // valid even if a wait times out first
     *q.abort_flag = 0;
     sm100::fence_mbar_init();
   }
 #define MCFFT_RQ_ALL(M)                                                                          \
   M(0) M(1) M(2) M(3) M(4) M(5) M(6) M(7) M(8) M(9) M(10) M(11) M(12) M(13) M(14) M(15) M(16)  \
   M(17) M(18) M(19) M(20) M(21)
-  auto tables = [&](int pi, uint32_t to) {
-    switch (a.pass[pi].variant) {
-#define MCFFT_RQ_TAB(V)                                                                      \
-  case V:                                                                                    \
-    queue_tables<typename PlainVariant<V, INV>::type>(a.pass[pi], smem + to, tid);           \
+  // the part of a pass's tables that depends on the plan
+  auto setup = [&](const RPass& P, uint32_t to) {
+    switch (P.variant) {
+#define MCFFT_RQ_TAB(V)                                                        \
+  case V:                                                                      \
+    PlainVariant<V, INV>::type::setup(P, smem + QueueShape::OFF_TAB + to, tid); \
     break;
       MCFFT_RQ_ALL(MCFFT_RQ_TAB)
       default: break;
     }
   };
   if (a.resident && tid < 512)
-    for (int pi = 0; pi < a.npass; ++pi) tables(pi, QueueShape::OFF_TAB + a.pass[pi].tw_off);
+    for (int pi = 0; pi < a.npass; ++pi) {
+      const RPass& P = a.pass[pi];
+      TabState::copy(P, base_u + QueueShape::OFF_TAB + P.tw_off, tid);
+      setup(P, P.tw_off);
+    }
+  asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
   const uint32_t G = gridDim.x, nlocal = a.nitems > blockIdx.x ? (a.nitems - blockIdx.x + G - 1) / G : 0;
   if (warp >= 16) {
@@ -330,26 +368,36 @@ __global__ void __launch_bounds__(640, 1) fft_reg_queue(const __grid_constant__ 
     asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
     const Sync<512> sync{1};
     const MmaFrags fr(a, tid);
-    int cur = -1;
-    uint32_t k = 0;
-    if (nlocal) wait_or_abort(&q.full[0], 0u, q.abort_flag);
-    while (k < nlocal) {
-      const int pi = (int)q.ring[2 * (k % NBUF)];
-      const RPass& P = a.pass[pi];
-      const uint32_t off = QueueShape::OFF_TAB + (a.resident ? P.tw_off : 0u), tab = base_u + off;
-      if (!a.resident && pi != cur) {
-        sync.group();  // nobody reads the old tables any more
-        tables(pi, off);
+    TabState ts;
+    QueuePlace pl(a, nlocal);
+    while (pl.k < nlocal) {
+      const RPass& P = a.pass[pl.it.pass];
+      if (a.resident) {
+        ts.off = P.tw_off;
+      } else {
+        // The barrier of the last switch: nobody reads the table before the
+        // current one any more, whose end of the area this one takes.
+        const bool fits = ts.fits(P) && pl.k > 0;  // copied already
+        const uint32_t off = ts.next_off(P);
+        if (!fits) {
+          sync.group();
+          TabState::copy(P, base_u + QueueShape::OFF_TAB + off, tid);
+        }
+        setup(P, off);
+        asm volatile("cp.async.wait_all;" ::: "memory");
         sync.group();
-        cur = pi;
+        ts.off = off;
+        ts.size = P.tab_bytes;
+        ts.end ^= 1u;
       }
+      const uint32_t tab = base_u + QueueShape::OFF_TAB + ts.off;
       switch (P.variant) {
-#define MCFFT_RQ_RUN(V)                                                                                 \
-  case V:                                                                                               \
-    k = queue_run<typename PlainVariant<V, INV>::type>(P, pi, fr, q, tab, tid, k, nlocal, sync);        \
+#define MCFFT_RQ_RUN(V)                                                                       \
+  case V:                                                                                     \
+    queue_run<typename PlainVariant<V, INV>::type>(a, P, fr, q, tab, ts, tid, pl, sync);      \
     break;
         MCFFT_RQ_ALL(MCFFT_RQ_RUN)
-        default: k = nlocal; break;
+        default: pl.k = nlocal; break;
       }
     }
   }
