@@ -1,7 +1,7 @@
 // fft_reg.cuh -- TMA-fed FFT pass kernel whose butterflies stay in registers.
 //
-// Persistent, one CTA per SM (small tiles: three); a tile holds C columns x L points, L = R1 R2,
-// both radices at most 32.  A thread holds 32 points of the tile in FP32: one
+// Persistent, one CTA per SM (small tiles: three); a tile holds C columns x L
+// points, L = R1 R2, both radices at most 32.  A thread holds 32 points of the tile in FP32: one
 // 32-point vector, two of 16 or four of 8 (fft_codelets.cuh), so a pass of up
 // to 1024 points is two phases with one exchange through shared memory:
 //
@@ -19,9 +19,10 @@
 // is too small a contraction to pay for staging its operand.  Measured on a
 // B200 (2^20 x 64, FP16 in, FP32 out, whole exec): 512 us with the tcgen05
 // split tiles, 375 us here; the same TMA copies without any arithmetic take
-// 350 us.  3D 256^3 FP32: 195 -> 141 us; plain 2^20 x 64: 255 -> 245 us (its
-// 16K points of arithmetic per 64 KB tile, 4.3 K cycles of the FP32 pipe, no
-// longer hide behind the copies).
+// 350 us.  3D 256^3 FP32: 195 -> 141 us.  Plain, where a 64 KB tile holds 16K
+// points, 4.3 K cycles of the FP32 pipe that no longer hide behind the copies:
+// 2D 1024^2 x 16 70.9 -> 65.6 us, 3D 256^3 92.3 -> 84.3, so 256 to 1024 plain
+// points are MmaPass (fft_mma.cuh: 57.1 and 72.4).
 //
 // Exchange in place.  Phase 1 writes its outputs into the slots its own warp
 // has read (k1 in the place of n1, lanes of the warp permuted so that phase 2
@@ -592,9 +593,14 @@ __global__ void __launch_bounds__(P::THREADS, P::MINB) fft_reg(const __grid_cons
     sm100::mbar_arrive_expect_tx(&full[i % NFULL], a.in_tile_bytes);
     tile::tma_load(&a.tmap_in, a.in_ndims, crd, base_u + b * P::BUF, &full[i % NFULL]);
   };
-  // The first loads are issued before the tables are in place.  Under a
-  // programmatic dependent launch the buffers the passes share are touched
-  // only after the wait; the tables are this launch's own constants.
+  // Small tiles: the first loads are issued before the tables are in place.
+  // Large ones issue them after the barrier, all from the one loop that holds
+  // the copying thread's state: with a second copy of the load before the
+  // barrier, and with the copying warps returning early instead of joining the
+  // consumers at the end, the consumers' code got slower (1024 x 16384 28.9 ->
+  // 32.5 us, 3D 256^3 68.9 -> 74.0, 2^20 x 64 213 -> 224, same registers).
+  // Under a programmatic dependent launch the buffers the passes share are
+  // touched only after the wait; the tables are this launch's own constants.
   uint32_t loaded = 0;
   if (producer) {
     if (lane == 0) {
@@ -604,8 +610,10 @@ __global__ void __launch_bounds__(P::THREADS, P::MINB) fft_reg(const __grid_cons
       for (int b = 0; b < NBUF; ++b) sm100::mbar_init(&done[b], NW);
       *abort_flag = 0;
       sm100::fence_mbar_init();
-      sm100::grid_dep_wait();
-      for (; loaded < mine && loaded < NBUF; ++loaded) load(loaded);
+      if constexpr (!P::BIG) {
+        sm100::grid_dep_wait();
+        for (; loaded < mine && loaded < NBUF; ++loaded) load(loaded);
+      }
     }
     __syncwarp();
   } else if (warp < NG * NW) {
@@ -620,6 +628,8 @@ __global__ void __launch_bounds__(P::THREADS, P::MINB) fft_reg(const __grid_cons
     if constexpr (P::BIG) asm volatile("setmaxnreg.dec.sync.aligned.u32 24;");
     if (producer && lane == 0) {
       uint32_t i = 0;
+      if constexpr (P::BIG)
+        for (; loaded < mine && loaded < NBUF; ++loaded) load(loaded);
       for (; i < mine; ++i) {
         const uint32_t b = i % NBUF;
         wait_or_abort(&done[b], (i / NBUF) & 1u, abort_flag);
@@ -639,10 +649,7 @@ __global__ void __launch_bounds__(P::THREADS, P::MINB) fft_reg(const __grid_cons
       for (; i < loaded; ++i) sm100::mbar_wait_bounded(&full[i % NFULL], (i / NFULL) & 1u, kWaitLimit);
     }
     __syncwarp();
-    __syncthreads();
-    return;  // the rest belongs to the warps that hold registers for it
-  }
-  {
+  } else {
     if constexpr (P::BIG) asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
     const int grp = NG == 1 ? 0 : tid / T, t = tid - grp * T;
     const Sync<T> sync{1 + grp};
