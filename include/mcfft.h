@@ -25,8 +25,9 @@
  *                     radix-16 stage scaled by 1/16 (radix-R tail by 1/R),
  *                     so out = DFT(in) * 2^scale_log2 with scale_log2 =
  *                     -log2(number of points of one transform).
- *   MCFFT_PREC_SPLIT  split hi+lo FP16 operands, three products per stage,
- *                     FP32 accumulation: FP32 in (or FP16 in with
+ *   MCFFT_PREC_SPLIT  FP32 arithmetic in registers, on lengths without such
+ *                     a pass split hi+lo FP16 operands, three products per
+ *                     stage, FP32 accumulation: FP32 in (or FP16 in with
  *                     MCFFT_FLAG_INPUT_F16), FP32 out, unnormalised DFT
  *                     (scale_log2 = 0), like FFTW_FORWARD/FFTW_BACKWARD.
  *

@@ -406,6 +406,13 @@ bool small_tiles(const mcfftPlan p, const PassSpec& s) {
 // per CTA slot the copying warps' run-ahead is worth more than the short start.
 int64_t direct_tiles(const mcfftPlan p) { return int64_t(p->split ? 6 : 16) * p->sms; }
 
+// MCFFT_FUSED=1: the fused four-step kernels (fused_for), which hold tcgen05
+// tiles.
+bool fused_wanted() {
+  const char* e = std::getenv("MCFFT_FUSED");
+  return e && std::atoi(e) != 0;
+}
+
 // Builds a pass on the TMA-fed kernel.  Returns MCFFT_UNSUPPORTED_SIZE when
 // the shape is outside what that kernel handles (the caller falls back).
 mcfftResult add_tile_pass(mcfftPlan p, const PassSpec& s, int only_tile_points = 0) {
@@ -440,7 +447,7 @@ mcfftResult add_tile_pass(mcfftPlan p, const PassSpec& s, int only_tile_points =
   // register passes or none.
   const int small = small_tiles(p, s) && !only_tile_points && !p->reg_queue ? 4096 : 0;
   for (int oi = small ? -1 : 0; oi < 2 && !k; ++oi) {
-    if (!p->reg_queue && (p->queue_planned || indexed)) break;
+    if (!p->reg_queue && (p->queue_planned || indexed || fused_wanted())) break;
     const TileKernel* cand = find_reg_kernel((int)s.L, ik, ok, s.posttw, p->split,
                                              oi < 0 ? small : order[oi], s.in_f16 != 0);
     if (!cand || (s.ncols + cand->C - 1) / cand->C * s.nouter >= (int64_t(1) << 31)) continue;
@@ -1431,8 +1438,7 @@ QPassAux make_aux(mcfftPlan p, size_t i, bool* any) {
 // intermediate is still in L2).  Off by default: on the 2^20 x 64 workload
 // the two pass launches measured faster (0.258 against 0.294 ms).
 const FusedKernel* fused_for(mcfftPlan p) {
-  const char* e = std::getenv("MCFFT_FUSED");
-  if (!e || std::atoi(e) == 0) return nullptr;
+  if (!fused_wanted()) return nullptr;
   if (p->ngroups != 1 || p->passes.size() != 2 || p->no_queue) return nullptr;
   const Pass &a = p->passes[0], &b = p->passes[1];
   if (!a.tiled || !b.tiled || !a.spec.posttw || b.spec.posttw || a.out_buf != kScratch ||
@@ -2115,7 +2121,7 @@ mcfftResult mcfftPlanCreateBatch(mcfftPlan* plan, const mcfftDesc* descs, int co
   // Plain plans first try the one-launch kernel on the register passes, then
   // the batch kernel.
   const bool reg = precision == MCFFT_PREC_FP16 && !std::getenv("MCFFT_QUEUE") &&
-                   !std::getenv("MCFFT_TILE_POINTS") && !std::getenv("MCFFT_NO_TILE");
+                   !std::getenv("MCFFT_TILE_POINTS") && !std::getenv("MCFFT_NO_TILE") && !fused_wanted();
   for (int bs = by_shape ? 1 : 0; bs >= 0; --bs) {
     bool indexed = false;
     mcfftResult r = MCFFT_UNSUPPORTED_SIZE;
