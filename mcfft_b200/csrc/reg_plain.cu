@@ -1,7 +1,8 @@
 // reg_plain.cu -- plain-form (FP16) register pass kernels, 16K-point tiles
 // (4096 points for small batches of rows):
-// 64 and 128 points as two register phases (RegPass), 256 to 1024 with the
-// radix-16 stages on the tensor cores (MmaPass).
+// 64 and 128 points as two register phases (RegPass), 256 to 1024 and rows of
+// 2048 and 4096 with the radix-16 stages on the tensor cores (MmaPass,
+// Mma2048, Mma4096).
 #include "reg_pass.h"
 
 namespace mcfft {
