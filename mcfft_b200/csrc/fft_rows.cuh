@@ -17,9 +17,9 @@
 //
 // 2048 points (plain form): 16 x 16 x 8, two phases as MmaPass with the
 // radix-8 step in registers, eight transforms per 16K-point tile.  Bound by
-// HBM from a few thousand transforms: 20000 in 70.3 us (4.7 TB/s), 79.5 on the
-// tcgen05 tile of four columns; 3000 in 18.5 against 23.6 us; as the rows of
-// 2048^2 x 4, 65.1 against 73.7 us in all.
+// HBM from a few thousand transforms: 20000 in 61 us (5.4 TB/s), 80 on the
+// tcgen05 tile of eight columns; 3000 in 15 against 24 us; as the rows of
+// 2048^2 x 4, 64 against 74 us in all.
 #pragma once
 #include "fft_mma.cuh"
 
