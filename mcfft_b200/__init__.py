@@ -166,6 +166,11 @@ class Plan:
         return inf
 
     def exec_ptr(self, in_ptr: int, out_ptr: int, direction: int = FORWARD, stream: int = 0):
+        # ctypes would take the address of bytes, strings and arrays for a
+        # pointer: anything but a plain integer goes through c_void_p, which
+        # refuses those (TypeError)
+        if not (type(in_ptr) is int and type(out_ptr) is int and type(stream) is int):
+            in_ptr, out_ptr, stream = (ctypes.c_void_p(v) for v in (in_ptr, out_ptr, stream))
         _check(lib().mcfftExec(self._h, in_ptr, out_ptr, direction, stream), "mcfftExec")
 
     def exec_host_ptr(self, in_ptr: int, out_ptr: int, direction: int = FORWARD, stream: int = 0):
