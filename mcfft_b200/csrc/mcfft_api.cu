@@ -429,7 +429,8 @@ mcfftResult add_tile_pass(mcfftPlan p, const PassSpec& s, int only_tile_points =
   // layout is missing; split form 8K points (its FP32 staging is twice as
   // large per point).
   int first = 16384;
-  if (const char* e = std::getenv("MCFFT_TILE_POINTS")) first = std::atoi(e);
+  const char* tile_env = std::getenv("MCFFT_TILE_POINTS");
+  if (tile_env) first = std::atoi(tile_env);
   int order[2] = {p->split ? 8192 : first, p->split ? 8192 : (first == 16384 ? 8192 : 16384)};
   if (only_tile_points) order[0] = order[1] = only_tile_points;
   const int in_elem = s.in_f16 ? 4 : 8, out_elem = s.out_f16 ? 4 : 8;
@@ -444,9 +445,11 @@ mcfftResult add_tile_pass(mcfftPlan p, const PassSpec& s, int only_tile_points =
   // on four-step, 2D and 3D transforms, plain 1.04x .. 1.13x).  Passes of the
   // batch queue, longer columns and the plain form's 8K-point tiles (small
   // batches) take the tcgen05 tiles; those of the one-launch kernel are
-  // register passes or none.
-  const int small = small_tiles(p, s) && !only_tile_points && !p->reg_queue ? 4096 : 0;
-  for (int oi = small ? -1 : 0; oi < 2 && !k; ++oi) {
+  // register passes or none.  A size that MCFFT_TILE_POINTS names is the only
+  // one tried here: the tcgen05 tiles of that size come before register
+  // passes of another.
+  const int small = small_tiles(p, s) && !only_tile_points && !tile_env && !p->reg_queue ? 4096 : 0;
+  for (int oi = small ? -1 : 0; oi < (tile_env ? 1 : 2) && !k; ++oi) {
     if (!p->reg_queue && (p->queue_planned || indexed || fused_wanted())) break;
     const TileKernel* cand = find_reg_kernel((int)s.L, ik, ok, s.posttw, p->split,
                                              oi < 0 ? small : order[oi], s.in_f16 != 0);
