@@ -1727,6 +1727,27 @@ mcfftResult exec_queue(mcfftPlan p, const void* in, void* out, int dir, cudaStre
   return MCFFT_SUCCESS;
 }
 
+// MCFFT_DEBUG_PLAN: what the finished plan runs, a line for the plan and one
+// per pass.
+void print_route(const mcfftPlan p) {
+  const char* how = !p->q.on        ? "pass by pass"
+                    : p->q.fused    ? "one launch, fused kernel"
+                    : !p->q.reg     ? "one launch, batch kernel"
+                    : p->q.resident ? "one launch, register passes, tables resident"
+                                    : "one launch, register passes, tables reloaded";
+  fprintf(stderr, "[mcfft] plan: %d groups, %zu passes, %s\n", p->ngroups, p->passes.size(), how);
+  for (size_t i = 0; i < p->passes.size(); ++i) {
+    const Pass& ps = p->passes[i];
+    if (!ps.tiled) {
+      fprintf(stderr, "[mcfft] pass %zu: L=%d, direct load\n", i, ps.k->L);
+      continue;
+    }
+    const TileKernel& k = *ps.tp.k;
+    fprintf(stderr, "[mcfft] pass %zu: L=%d, %s, %d-point tiles%s\n", i, k.L,
+            k.reg_kind >= 0 ? "register" : "tcgen05", k.tile_points, ps.tp.small ? ", no TMA" : "");
+  }
+}
+
 mcfftResult plan_finish(mcfftPlan p, mcfftPlan* out) {
   mcfftResult r = MCFFT_SUCCESS;
   if (p->reg_queue) r = build_reg_queue(p);
@@ -1746,6 +1767,7 @@ mcfftResult plan_finish(mcfftPlan p, mcfftPlan* out) {
     p->info.ctas = p->q.on ? p->q.grid : (f.tiled ? f.tp.grid : f.grid);
   }
   p->info.workspace_bytes = (int64_t)p->scratch_bytes;
+  if (std::getenv("MCFFT_DEBUG_PLAN")) print_route(p);
   *out = p;
   return MCFFT_SUCCESS;
 }

@@ -1,5 +1,7 @@
 """Which kernels a plan runs: switches and rules that choose between kernel
 families, seen in the plan's information rather than in its results."""
+import math
+
 import pytest
 
 torch = pytest.importorskip("torch")
@@ -42,3 +44,83 @@ def test_tile_points_switch_split(n, batch, monkeypatch):
         assert p.info().tile_points == 8192
         y, _ = run(p, x, False)
     assert compare(y, oracle.fft1d(rounded(x, False)))[0] < SPLIT_TOL
+
+
+def _route(capfd, monkeypatch, make):
+    """The plan's line and its passes' lines as MCFFT_DEBUG_PLAN prints them."""
+    monkeypatch.setenv("MCFFT_DEBUG_PLAN", "1")
+    capfd.readouterr()
+    with make():
+        pass
+    lines = capfd.readouterr().err.splitlines()
+    plan = [ln for ln in lines if ln.startswith("[mcfft] plan: ")]
+    passes = [ln.split(": ", 1)[1] for ln in lines if ln.startswith("[mcfft] pass ")]
+    assert len(plan) == 1, lines
+    return plan[0].split("passes, ", 1)[1], passes
+
+
+@pytest.mark.parametrize("shape,batch,prec,expect", [
+    # few rows: 4096-point tiles without TMA; more: with TMA; many: full tiles
+    ((1024,), 8, mc.PREC_FP16, ["L=1024, register, 4096-point tiles, no TMA"]),
+    ((4096,), 256, mc.PREC_FP16, ["L=4096, register, 4096-point tiles, no TMA"]),
+    ((4096,), 4000, mc.PREC_FP16, ["L=4096, register, 4096-point tiles"]),
+    ((1024,), 16384, mc.PREC_FP16, ["L=1024, register, 16384-point tiles"]),
+    ((64,), 3, mc.PREC_SPLIT, ["L=64, register, 4096-point tiles, no TMA"]),
+    ((4096,), 1000, mc.PREC_SPLIT, ["L=4096, register, 4096-point tiles"]),
+    ((1024,), 16384, mc.PREC_SPLIT, ["L=1024, register, 8192-point tiles"]),
+    ((2048,), 5001, mc.PREC_FP16, ["L=2048, register, 16384-point tiles"]),
+    ((1024, 1024), 16, mc.PREC_FP16, ["L=1024, register, 16384-point tiles"] * 2),
+    ((1 << 18,), 30, mc.PREC_SPLIT, ["L=512, register, 8192-point tiles"] * 2),
+    # lengths without a register routine
+    ((32,), 512, mc.PREC_FP16, ["L=32, tcgen05, 8192-point tiles"]),
+    ((8192,), 8, mc.PREC_FP16, ["L=8192, tcgen05, 16384-point tiles"]),
+    ((2048,), 8, mc.PREC_SPLIT, ["L=2048, tcgen05, 8192-point tiles"])])
+def test_pass_kernels(shape, batch, prec, expect, capfd, monkeypatch):
+    monkeypatch.setenv("MCFFT_AUTOTUNE", "0")
+    how, passes = _route(capfd, monkeypatch, lambda: mc.Plan(shape, batch, prec))
+    assert how == "pass by pass"
+    assert passes == expect
+
+
+def _descs(shapes, mixed):
+    """One descriptor per transform, back to back; mixed: outputs in the
+    opposite order."""
+    items = [s for s, c in shapes for _ in range(c)]
+    size = [math.prod(s) for s in items]
+    total, at, descs = sum(size), 0, []
+    for s, n in zip(items, size):
+        descs.append((s, 1, at, total - at - n if mixed else at))
+        at += n
+    return descs
+
+
+ALL = [((64,), 1), ((128,), 300), ((256,), 67), ((512,), 33), ((1024,), 17), ((2048,), 9), ((4096,), 5),
+       ((1 << 13,), 3), ((1 << 14,), 3), ((1 << 15,), 2), ((1 << 17,), 2), ((1 << 18,), 1), ((1 << 20,), 1),
+       ((1 << 19,), 1), ((64, 2048), 3), ((64, 64), 3), ((128, 1024), 2), ((512, 256), 2), ((1024, 512), 1),
+       ((64, 64, 128), 1)]
+LONG = [s for s in ALL if s[0] not in ((64,), (128,), (64, 64))]
+
+
+@pytest.mark.parametrize("shapes,mixed,prec,expect", [
+    (ALL, False, mc.PREC_FP16, "register passes, tables reloaded"),
+    (LONG, False, mc.PREC_FP16, "register passes, tables reloaded"),
+    (LONG, True, mc.PREC_FP16, "register passes, tables reloaded"),
+    ([((256,), 65), ((512,), 1)], False, mc.PREC_FP16, "register passes, tables resident"),
+    ([((256,), 65), ((512,), 1)], True, mc.PREC_FP16, "register passes, tables resident"),
+    # the batch of the timeout test
+    ([((256,), 3), ((4096,), 2), ((1 << 16,), 1), ((128, 256), 1)], False, mc.PREC_FP16,
+     "register passes, tables reloaded"),
+    # no routine: 1D lengths of 64 and 128 points at unrelated offsets, a side
+    # of 32, rows of 2048 as a second pass, the split form
+    ([((128,), 3), ((256,), 3)], True, mc.PREC_FP16, "batch kernel"),
+    ([((256,), 3), ((32, 256), 1)], False, mc.PREC_FP16, "batch kernel"),
+    ([((256,), 3), ((1 << 21,), 1)], False, mc.PREC_FP16, "batch kernel"),
+    ([((256,), 3), ((512,), 1)], False, mc.PREC_SPLIT, "batch kernel")])
+def test_uneven_kernels(shapes, mixed, prec, expect, capfd, monkeypatch):
+    """The lists of the uneven parity tests among them, which cannot tell the
+    two one-launch kernels apart."""
+    monkeypatch.setenv("MCFFT_AUTOTUNE", "0")
+    how, passes = _route(capfd, monkeypatch, lambda: mc.Plan(descs=_descs(shapes, mixed), precision=prec))
+    assert how == "one launch, " + expect
+    family = "register" if "register" in expect else "tcgen05"
+    assert all(family in p for p in passes), passes
