@@ -1024,6 +1024,7 @@ mcfftResult plan_begin(mcfftPlan* out, mcfftPrecision prec, unsigned flags, mcff
   }
   mcfftPlan p = new (std::nothrow) mcfftPlan_st();
   if (!p) return MCFFT_ALLOC_FAILED;
+  if (std::getenv("MCFFT_DEBUG_PLAN")) fprintf(stderr, "[mcfft] begin plan\n");
   cudaGetDevice(&p->device);
   cudaDeviceGetAttribute(&p->sms, cudaDevAttrMultiProcessorCount, p->device);
   p->split = prec == MCFFT_PREC_SPLIT;
@@ -2006,14 +2007,61 @@ extern "C" {
 namespace mcfft {
 namespace {
 
+// Transforms of one shape: per-transform input and output offsets; affine:
+// they follow each other in both buffers.
+struct BatchGroup {
+  mcfftDesc shape;
+  std::vector<int64_t> in, out;
+  bool affine = true;
+};
+
+// Whether the one-launch kernel on the register passes has a routine for
+// every pass of the groups (a plan it cannot take after all, for instance
+// for its offsets, is refused while it is built).  A group's passes are those
+// of build_group_passes / build_indexed_group for a plan with reg_queue set.
+bool reg_queue_takes(const mcfftPlan p, const std::vector<BatchGroup>& groups) {
+  if (groups.size() < 2) return false;
+  auto has = [](int64_t L, layout::Kind ik, layout::Kind ok, bool posttw) {
+    if (L > kMaxTilePass) return false;
+    const TileKernel* k = find_reg_kernel((int)L, ik, ok, posttw, false, 16384, true);
+    return k && reg_queue_variant(*k) >= 0;
+  };
+  size_t passes = 0;
+  for (const BatchGroup& g : groups) {
+    const int64_t* d = g.shape.dims;
+    const int nd = g.shape.ndim;
+    for (int k = 0; k < nd; ++k)
+      if (!is_pow2(d[k])) return false;
+    bool ok;
+    if (nd > 1) {
+      ok = has(d[nd - 1], layout::ROW, layout::ROW, false);
+      for (int k = 0; k + 1 < nd; ++k) ok = ok && has(d[k], layout::COL, layout::COL, false);
+      passes += nd;
+    } else if (d[0] <= max_one_pass(p)) {
+      // at unrelated offsets only the tensor-core rows (reg_gather_staging)
+      ok = (g.affine || d[0] >= 256) && has(d[0], layout::ROW, layout::ROW, false);
+      passes += 1;
+    } else if (std::getenv("MCFFT_FOURSTEP_N1")) {
+      ok = true;  // found out while the plan is built
+      passes += 2;
+    } else {
+      const int64_t n1 = int64_t(1) << default_lg1(p, d[0]);
+      ok = has(n1, layout::COL, layout::COL, true) && has(d[0] / n1, layout::ROW, layout::COL, false);
+      passes += 2;
+    }
+    if (!ok) return false;
+  }
+  return passes <= (size_t)kRegQueueMaxPasses;
+}
+
 // The plan of a batch of descriptors.  by_shape: one group per shape
 // (indexed where its transforms are not contiguous and in order; *indexed
 // tells whether any was); else one group per run of consecutive
 // descriptors of one shape whose data follow each other in both buffers.
-// reg: for the one-launch kernel on the register passes, which takes plans of
-// several groups whose passes are all of its variants.
+// *reg: whether the plan may be one for the one-launch kernel on the register
+// passes; on return, whether it was built as one.
 mcfftResult create_batch(mcfftPlan* plan, const mcfftDesc* descs, int count,
-                         mcfftPrecision precision, unsigned flags, bool by_shape, bool reg,
+                         mcfftPrecision precision, unsigned flags, bool by_shape, bool* reg,
                          bool* indexed) {
   mcfftPlan p = nullptr;
   mcfftResult r = plan_begin(plan, precision, flags, &p);
@@ -2032,24 +2080,18 @@ mcfftResult create_batch(mcfftPlan* plan, const mcfftDesc* descs, int count,
     const int64_t len = g.batch * points(g);
     return same && d.in_offset == g.in_offset + len && d.out_offset == g.out_offset + len;
   };
-  // Groups: (shape, per-transform input and output offsets) in order of
-  // first appearance.
-  struct Group {
-    mcfftDesc shape;
-    std::vector<int64_t> in, out;
-  };
-  std::vector<Group> groups;
+  std::vector<BatchGroup> groups;  // in order of first appearance
   if (by_shape) {
     for (int i = 0; i < count; ++i) {
       const mcfftDesc& d = descs[i];
-      Group* g = nullptr;
+      BatchGroup* g = nullptr;
       for (auto& x : groups) {
         bool same = x.shape.ndim == d.ndim;
         for (int k = 0; k < d.ndim && same; ++k) same = x.shape.dims[k] == d.dims[k];
         if (same) g = &x;
       }
       if (!g) {
-        groups.push_back(Group{d, {}, {}});
+        groups.push_back(BatchGroup{d, {}, {}});
         g = &groups.back();
       }
       const int64_t n = points(d);
@@ -2059,7 +2101,7 @@ mcfftResult create_batch(mcfftPlan* plan, const mcfftDesc* descs, int count,
       }
     }
     // groups are independent: queue them by dimensionality, then shape
-    std::stable_sort(groups.begin(), groups.end(), [](const Group& a, const Group& b) {
+    std::stable_sort(groups.begin(), groups.end(), [](const BatchGroup& a, const BatchGroup& b) {
       if (a.shape.ndim != b.shape.ndim) return a.shape.ndim < b.shape.ndim;
       for (int k = 0; k < a.shape.ndim; ++k)
         if (a.shape.dims[k] != b.shape.dims[k]) return a.shape.dims[k] < b.shape.dims[k];
@@ -2070,7 +2112,7 @@ mcfftResult create_batch(mcfftPlan* plan, const mcfftDesc* descs, int count,
       mcfftDesc g = descs[i];
       for (++i; i < count && continues(i, g); ++i) g.batch += descs[i].batch;
       const int64_t n = points(g);
-      Group x{g, {}, {}};
+      BatchGroup x{g, {}, {}};
       for (int64_t b = 0; b < g.batch; ++b) {
         x.in.push_back(g.in_offset + b * n);
         x.out.push_back(g.out_offset + b * n);
@@ -2078,18 +2120,24 @@ mcfftResult create_batch(mcfftPlan* plan, const mcfftDesc* descs, int count,
       groups.push_back(x);
     }
   }
+  for (BatchGroup& g : groups) {
+    const int64_t n = points(g.shape);
+    for (size_t b = 0; b < g.in.size() && g.affine; ++b)
+      g.affine = g.in[b] == g.in[0] + (int64_t)b * n && g.out[b] == g.out[0] + (int64_t)b * n;
+  }
   p->queue_planned = groups.size() > 1;
-  p->reg_queue = reg && p->queue_planned;
-  if (reg && !p->reg_queue) r = MCFFT_UNSUPPORTED_SIZE;
+  // Asked before anything is built: plans built for that kernel and then
+  // refused were built twice (with recorded tuning, all plain single shapes:
+  // 1024 x 8 3.5 ms against 2.9, 2^20 x 64 6.6 against 6.0; an uneven batch
+  // with a side of 32 20 against 18).
+  p->reg_queue = *reg;
+  p->reg_queue = *reg = *reg && reg_queue_takes(p, groups);
   if (const char* e = std::getenv("MCFFT_QUEUE")) p->queue_planned = std::atoi(e) != 0;
   for (size_t gi = 0; gi < groups.size() && !r; ++gi) {
-    const Group& g = groups[gi];
+    const BatchGroup& g = groups[gi];
     const int64_t n = points(g.shape), B = (int64_t)g.in.size();
-    bool affine = true;
-    for (int64_t b = 0; b < B && affine; ++b)
-      affine = g.in[b] == g.in[0] + b * n && g.out[b] == g.out[0] + b * n;
     int sl = 0;
-    if (affine) {
+    if (g.affine) {
       r = build_group(p, g.shape.ndim, g.shape.dims, B, g.in[0], g.out[0], &sl);
     } else {
       *indexed = true;
@@ -2148,12 +2196,11 @@ mcfftResult mcfftPlanCreateBatch(mcfftPlan* plan, const mcfftDesc* descs, int co
   const bool reg = precision == MCFFT_PREC_FP16 && !std::getenv("MCFFT_QUEUE") &&
                    !std::getenv("MCFFT_TILE_POINTS") && !std::getenv("MCFFT_NO_TILE") && !fused_wanted();
   for (int bs = by_shape ? 1 : 0; bs >= 0; --bs) {
-    bool indexed = false;
-    mcfftResult r = MCFFT_UNSUPPORTED_SIZE;
-    if (reg) r = create_batch(plan, descs, count, precision, flags, bs != 0, true, &indexed);
-    if (r == MCFFT_UNSUPPORTED_SIZE) {
-      indexed = false;
-      r = create_batch(plan, descs, count, precision, flags, bs != 0, false, &indexed);
+    bool indexed = false, as_reg = reg;
+    mcfftResult r = create_batch(plan, descs, count, precision, flags, bs != 0, &as_reg, &indexed);
+    if (r == MCFFT_UNSUPPORTED_SIZE && as_reg) {
+      indexed = as_reg = false;
+      r = create_batch(plan, descs, count, precision, flags, bs != 0, &as_reg, &indexed);
     }
     if (bs == 0 || r != MCFFT_UNSUPPORTED_SIZE || !indexed) return r;
   }

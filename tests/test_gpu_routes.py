@@ -124,3 +124,26 @@ def test_uneven_kernels(shapes, mixed, prec, expect, capfd, monkeypatch):
     assert how == "one launch, " + expect
     family = "register" if "register" in expect else "tcgen05"
     assert all(family in p for p in passes), passes
+
+
+@pytest.mark.parametrize("make", [
+    lambda: mc.Plan((1024,), 8),
+    lambda: mc.Plan((256, 256), 3),
+    lambda: mc.Plan((1024,), 8, mc.PREC_SPLIT),
+    lambda: mc.Plan(descs=_descs([((256,), 3), ((512,), 2)], False)),
+    lambda: mc.Plan(descs=_descs([((128,), 3), ((256,), 3)], True)),
+    lambda: mc.Plan(descs=_descs([((256,), 3), ((32, 256), 1)], False)),
+    lambda: mc.Plan(descs=_descs([((256,), 3), ((1 << 21,), 1)], False)),
+    lambda: mc.Plan(descs=_descs([((64, 64, 64 << i), 1) for i in range(7)]
+                                 + [((64, 128, 64 << i), 1) for i in range(7)]
+                                 + [((64 << i, 64), 1) for i in range(5)], False))],
+    ids=["1d", "2d", "split", "uneven", "uneven_mixed_128", "uneven_side_32", "uneven_2p21", "uneven_52_passes"])
+def test_plan_built_once(make, capfd, monkeypatch):
+    """The choice between the one-launch kernels is made before anything is
+    built."""
+    monkeypatch.setenv("MCFFT_AUTOTUNE", "0")
+    monkeypatch.setenv("MCFFT_DEBUG_PLAN", "1")
+    capfd.readouterr()
+    with make():
+        pass
+    assert capfd.readouterr().err.count("[mcfft] begin plan") == 1
