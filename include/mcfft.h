@@ -204,7 +204,8 @@ MCFFT_API mcfftResult mcfftErrorNorms(const void* y, int y_f16, const void* ref,
  * reuse the record instead of timing.  Export writes this process's records
  * to a text file, Import reads such a file (adding to and replacing records;
  * a malformed file changes nothing and returns MCFFT_INVALID_VALUE), Forget
- * drops every record.  Records of another GPU model are kept but unused. */
+ * drops every record.  Records of another GPU model, or of other kernels (an
+ * older library, or another kernel family), are kept but unused. */
 MCFFT_API mcfftResult mcfftWisdomExport(const char* path);
 MCFFT_API mcfftResult mcfftWisdomImport(const char* path);
 MCFFT_API mcfftResult mcfftWisdomForget(void);

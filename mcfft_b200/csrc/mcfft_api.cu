@@ -648,9 +648,10 @@ float time_tile_pass(const TilePass& tp, void* a, void* b, cudaStream_t st) {
 
 // Autotuning records ("wisdom"): the tile shape the plan-time tuner chose
 // for a pass, keyed by the GPU (name and SM count) and everything the
-// choice depends on (the pass's length, layout, strides and extents).  The
-// records of this process can be written to a text file and read back by a
-// later process, whose plans then take the recorded shapes without timing.
+// choice depends on (the pass's length, layout, strides and extents, and the
+// kernels it was made among: kernels_key).  The records of this process can
+// be written to a text file and read back by a later process, whose plans
+// then take the recorded shapes without timing.
 // File format: the line "mcfft-wisdom 1", then one record per line:
 // "<gpu name>\t<sms>\t<pass key>\t<tile points>".
 struct Wisdom {
@@ -674,13 +675,26 @@ std::string gpu_key(const mcfftPlan p) {
   return name + "\t" + std::to_string(p->sms);
 }
 
-std::string pass_key(const PassSpec& s) {
+// The kernels a choice was made among: their generation, raised whenever the
+// kernels behind a recorded choice change (records of others are read and
+// kept, but match no plan), and the family a plan's passes may come from.  The
+// same pass is a register pass in one plan and a tcgen05 tile in another: a
+// choice between tcgen05 tiles says nothing about a register pass.
+constexpr int kKernelGeneration = 2;
+std::string kernels_key(const mcfftPlan p) {
+  std::string k = " g" + std::to_string(kKernelGeneration);
+  k += std::getenv("MCFFT_NO_TILE") ? " direct" : p->queue_planned ? " queue" : fused_wanted() ? " fused" : " register";
+  if (const char* e = std::getenv("MCFFT_TILE_POINTS")) k += " t" + std::to_string(std::atoi(e));
+  return k;
+}
+
+std::string pass_key(const mcfftPlan p, const PassSpec& s) {
   char b[512];
   std::snprintf(b, sizeof b, "L%lld c%d t%d i%lld,%lld,%lld o%lld,%lld,%lld n%lld,%lld h%d,%d N%lld",
                 (long long)s.L, (int)s.colfast, (int)s.posttw, (long long)s.in_sp, (long long)s.in_sc,
                 (long long)s.in_so, (long long)s.out_sp, (long long)s.out_sc, (long long)s.out_so,
                 (long long)s.ncols, (long long)s.nouter, s.in_f16, s.out_f16, (long long)s.postN);
-  return b;
+  return b + kernels_key(p);
 }
 
 int wisdom_find(const std::string& key) {
@@ -718,7 +732,7 @@ mcfftResult autotune_group(mcfftPlan p, size_t first, int64_t points) {
     // queue, which the tuner's single-pass timing does not model)
     if (!p->passes[i].tiled || p->passes[i].in_tab || p->passes[i].out_tab) continue;
     if (p->passes[i].tp.k->tile_points == 4096) continue;  // chosen by size (small_tiles)
-    const int rec = wisdom_find(gk + "\t" + pass_key(p->passes[i].spec));
+    const int rec = wisdom_find(gk + "\t" + pass_key(p, p->passes[i].spec));
     if (!rec) {
       todo.push_back(i);
       continue;
@@ -758,7 +772,7 @@ mcfftResult autotune_group(mcfftPlan p, size_t first, int64_t points) {
       p->passes[i] = cand;
     }
     if (t0 > 0.f && t1 > 0.f)
-      wisdom_put(gk + "\t" + pass_key(p->passes[i].spec), p->passes[i].tp.k->tile_points);
+      wisdom_put(gk + "\t" + pass_key(p, p->passes[i].spec), p->passes[i].tp.k->tile_points);
   }
   cudaFree(a);
   cudaFree(b);
@@ -1173,7 +1187,7 @@ int tune_fourstep(mcfftPlan p, int64_t n, int64_t batch, int64_t in_off, int64_t
   char kb[160];
   std::snprintf(kb, sizeof kb, "fourstep n%lld b%lld p%d f%u", (long long)n, (long long)batch,
                 (int)p->prec, p->flags);
-  const std::string key = gpu_key(p) + "\t" + kb;
+  const std::string key = gpu_key(p) + "\t" + kb + kernels_key(p);
   if (const int rec = wisdom_find(key)) return rec;
   // each candidate's passes are built, timed, then removed again
   const size_t first = p->passes.size();

@@ -147,3 +147,50 @@ def test_plan_built_once(make, capfd, monkeypatch):
     with make():
         pass
     assert capfd.readouterr().err.count("[mcfft] begin plan") == 1
+
+
+@pytest.fixture
+def no_records():
+    mc.wisdom_forget()
+    yield
+    mc.wisdom_forget()
+
+
+@pytest.mark.parametrize("shape,batch", [((1024, 1024), 16), ((1 << 20,), 4)])
+def test_records_of_other_kernels(shape, batch, no_records):
+    """The passes of a plan bound for the batch kernel (a side of 32) are
+    tcgen05 tiles; what its tuner records says nothing about a plan of the
+    same passes on register kernels, which is tuned by itself."""
+    with mc.Plan(shape, batch) as p:
+        alone = p.info().timed_passes
+    mc.wisdom_forget()
+    n = math.prod(shape) * batch
+    with mc.Plan(descs=[(shape, batch, 0, 0), ((32, 256), 1, n, n)]) as p:
+        assert p.info().timed_passes > 0
+    with mc.Plan(shape, batch) as p:
+        assert p.info().timed_passes == alone > 0
+    with mc.Plan(shape, batch) as p:
+        assert p.info().timed_passes == 0
+
+
+def test_records_of_older_kernels(no_records, tmp_path, capfd, monkeypatch):
+    """Records written before they named the kernels: read, but no plan
+    follows them (here they ask for 8K-point tiles and another split)."""
+    path = tmp_path / "w.txt"
+    with mc.Plan((1 << 20,), 64) as p:
+        alone = p.info().timed_passes
+    mc.wisdom_export(str(path))
+    old = []
+    for ln in path.read_text().splitlines()[1:]:
+        name, sms, key, _ = ln.split("\t")
+        old.append("\t".join([name, sms, key.split(" g")[0], "9" if key.startswith("fourstep") else "8192"]))
+    assert len(old) >= 3
+    path.write_text("\n".join(["mcfft-wisdom 1"] + old) + "\n")
+    mc.wisdom_forget()
+    mc.wisdom_import(str(path))
+    monkeypatch.setenv("MCFFT_DEBUG_PLAN", "1")
+    with mc.Plan((1 << 20,), 64) as p:
+        assert p.info().timed_passes == alone
+    assert "pass 0: L=1024, register, 16384-point tiles" in capfd.readouterr().err
+    mc.wisdom_export(str(path))  # kept beside the new ones
+    assert set(old) <= set(path.read_text().splitlines())
