@@ -88,18 +88,18 @@ __device__ __forceinline__ void dft4(T& ar, T& ai, T& br, T& bi, T& cr, T& ci, T
   }
 }
 
-template <int R, bool INV, class T, bool H16 = false>
+template <int R, bool INV, class T>
 struct Dft;
 
-template <bool INV, class T, bool H16>
-struct Dft<4, INV, T, H16> {
+template <bool INV, class T>
+struct Dft<4, INV, T> {
   static __device__ __forceinline__ void run(T (&re)[4], T (&im)[4]) {
     dft4<INV>(re[0], im[0], re[1], im[1], re[2], im[2], re[3], im[3]);
   }
 };
 
-template <bool INV, class T, bool H16>
-struct Dft<8, INV, T, H16> {
+template <bool INV, class T>
+struct Dft<8, INV, T> {
   // n = 4 m + j: radix 2 over m, twiddle W8^(j q), radix 4 over j
   static __device__ __forceinline__ void run(T (&re)[8], T (&im)[8]) {
     constexpr float h = 0.70710678118654752440f;
@@ -134,18 +134,12 @@ struct Dft<8, INV, T, H16> {
   }
 };
 
-// H16: the factors W16^(j q) rounded to FP16.  The radix-4 steps around them
-// are exact, so the result is the product with the FP16 DFT-16 matrix that
-// the tcgen05 tiles multiply by, to FP32 rounding: a plain-form pass gives
-// the same transform whichever of the two kernels the tuner picks.
-template <bool INV, class T, bool H16>
-struct Dft<16, INV, T, H16> {
+template <bool INV, class T>
+struct Dft<16, INV, T> {
   // n = 4 m + j: radix 4 over m for each j, twiddle W16^(j q), radix 4 over j
   static __device__ __forceinline__ void run(T (&re)[16], T (&im)[16]) {
     constexpr float s = INV ? 1.f : -1.f;
-    constexpr float c1 = H16 ? 0.923828125f : 0.92387953251128675613f;
-    constexpr float s1 = H16 ? 0.382568359375f : 0.38268343236508977173f;
-    constexpr float h = H16 ? 0.70703125f : 0.70710678118654752440f;
+    constexpr float c1 = 0.92387953251128675613f, s1 = 0.38268343236508977173f, h = 0.70710678118654752440f;
 #pragma unroll
     for (int j = 0; j < 4; ++j)
       dft4<INV>(re[j], im[j], re[j + 4], im[j + 4], re[j + 8], im[j + 8], re[j + 12], im[j + 12]);

@@ -264,7 +264,7 @@ struct RegPass {
           r[n] = pack2(a.x, b.x);
           i[n] = pack2(a.y, b.y);
         }
-        Dft<R, INV, P2, true>::run(r, i);
+        Dft<R, INV, P2>::run(r, i);
 #pragma unroll
         for (int k = 0; k < R; ++k) {
           re[j / 2 * R + k] = r[k];
