@@ -60,24 +60,24 @@ __global__ void __launch_bounds__(P::T, P::MINB) fft_small(const __grid_constant
   if constexpr (IsReg4096<P>::value) {
     sm100::grid_dep_launch();
     P::template phases<true>(base_u, base_u + P::BUF, t, in, out);
-    return;
-  }
+  } else {
 #pragma unroll
-  for (int i = 0; i < IN / 16 / T; ++i) {
-    const uint32_t o = (i * T + t) * 16, g = P::in_map(o);
-    const bool valid = g < n * P::EI;
-    cp_async16(base_u + o, in + (valid ? g : 0), valid);
-  }
-  asm volatile("cp.async.wait_all;" ::: "memory");
-  const typename P::State st(a, t);
-  sm100::grid_dep_launch();
-  __syncthreads();
-  P::run(a, st, base_u, base_u + P::BUF, t, 0, Sync<T>{1});
-  __syncthreads();
+    for (int i = 0; i < IN / 16 / T; ++i) {
+      const uint32_t o = (i * T + t) * 16, g = P::in_map(o);
+      const bool valid = g < n * P::EI;
+      cp_async16(base_u + o, in + (valid ? g : 0), valid);
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    const typename P::State st(a, t);
+    sm100::grid_dep_launch();
+    __syncthreads();
+    P::run(a, st, base_u, base_u + P::BUF, t, 0, Sync<T>{1});
+    __syncthreads();
 #pragma unroll 8
-  for (int i = 0; i < OUT / 16 / T; ++i) {
-    const uint32_t o = (i * T + t) * 16, g = P::out_map(o);
-    if (g < n * P::EO) *reinterpret_cast<uint4*>(out + g) = *reinterpret_cast<const uint4*>(smem + o);
+    for (int i = 0; i < OUT / 16 / T; ++i) {
+      const uint32_t o = (i * T + t) * 16, g = P::out_map(o);
+      if (g < n * P::EO) *reinterpret_cast<uint4*>(out + g) = *reinterpret_cast<const uint4*>(smem + o);
+    }
   }
 }
 
