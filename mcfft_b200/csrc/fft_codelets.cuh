@@ -1,5 +1,6 @@
-// fft_codelets.cuh -- register-resident DFTs of 4, 8, 16 and 32 points in
-// FP32, the arithmetic of the register pass kernels (fft_reg.cuh).
+// fft_codelets.cuh -- register-resident DFTs of 8 and 16 points in FP32, the
+// radix-4 step they share and the first step of a 32-point one: the arithmetic
+// of the register pass kernels (fft_reg.cuh).
 //
 // One source serves two number types: `float` (one transform per thread at a
 // time) and P2, a pair of FP32 lanes in one 64-bit register on which the
@@ -90,13 +91,6 @@ __device__ __forceinline__ void dft4(T& ar, T& ai, T& br, T& bi, T& cr, T& ci, T
 
 template <int R, bool INV, class T>
 struct Dft;
-
-template <bool INV, class T>
-struct Dft<4, INV, T> {
-  static __device__ __forceinline__ void run(T (&re)[4], T (&im)[4]) {
-    dft4<INV>(re[0], im[0], re[1], im[1], re[2], im[2], re[3], im[3]);
-  }
-};
 
 template <bool INV, class T>
 struct Dft<8, INV, T> {

@@ -126,10 +126,9 @@ struct RegPass {
   static constexpr int lc = lgC < 5 ? lgC : 5;  // lanes along columns (column passes)
   static_assert(KIND == kRR || 5 - lc >= h, "rows of one line sit in one warp");
   static constexpr int BUF = TP * (EI > EO ? EI : EO);
-  // Twiddle table: packed pairs (k, k + 1) of one vector (R1 = 32) or one
-  // factor doubled for two columns, 16 bytes; FP32 form 8 bytes.
-  static constexpr int TWN = PK ? (R1 == 32 ? L / 2 : L) : L;  // entries, k-major, v fastest
-  static constexpr int TWB = TWN * (PK ? 16 : 8);
+  // Twiddle table, k-major, v fastest: one factor doubled for two columns, 16
+  // bytes; FP32 form 8 bytes.
+  static constexpr int TWB = L * (PK ? 16 : 8);
   static constexpr int NG = T >= 256 ? 512 / T : 1;  // tiles in work at a time
   static constexpr int NBUF = T >= 256 ? 3 : 2;
   // Load barriers: a ring long enough that one group alone waits on each
@@ -240,36 +239,24 @@ struct RegPass {
 
   // --------------------------------------------------------- plain, packed
   // R-point DFTs of this thread's 32 points, in FP16 words w[j][n] and out in
-  // packed FP32 pairs: R = 32, pair i = outputs (2i, 2i + 1) of the one
-  // vector; else pair (j / 2, k) = output k of vectors j and j + 1.
+  // packed FP32 pairs: pair (j / 2, k) = output k of vectors j and j + 1.
   template <int R>
   static __device__ __forceinline__ void dft_pk(const uint32_t (&w)[32 / R][R], P2 (&re)[16], P2 (&im)[16]) {
-    if constexpr (R == 32) {
+    static_assert(R <= 16, "two vectors per thread");
 #pragma unroll
-      for (int n = 0; n < 16; ++n) {
-        const float2 x0 = sm100::unpack_half2(w[0][n]), x1 = sm100::unpack_half2(w[0][n + 16]);
-        float er, ei, odr, odi;
-        split32<INV>(x0.x, x0.y, x1.x, x1.y, n, er, ei, odr, odi);
-        re[n] = pack2(er, odr);
-        im[n] = pack2(ei, odi);
+    for (int j = 0; j < 32 / R; j += 2) {
+      P2 r[R], i[R];
+#pragma unroll
+      for (int n = 0; n < R; ++n) {
+        const float2 a = sm100::unpack_half2(w[j][n]), b = sm100::unpack_half2(w[j + 1][n]);
+        r[n] = pack2(a.x, b.x);
+        i[n] = pack2(a.y, b.y);
       }
-      Dft<16, INV, P2>::run(re, im);
-    } else {
+      Dft<R, INV, P2>::run(r, i);
 #pragma unroll
-      for (int j = 0; j < 32 / R; j += 2) {
-        P2 r[R], i[R];
-#pragma unroll
-        for (int n = 0; n < R; ++n) {
-          const float2 a = sm100::unpack_half2(w[j][n]), b = sm100::unpack_half2(w[j + 1][n]);
-          r[n] = pack2(a.x, b.x);
-          i[n] = pack2(a.y, b.y);
-        }
-        Dft<R, INV, P2>::run(r, i);
-#pragma unroll
-        for (int k = 0; k < R; ++k) {
-          re[j / 2 * R + k] = r[k];
-          im[j / 2 * R + k] = i[k];
-        }
+      for (int k = 0; k < R; ++k) {
+        re[j / 2 * R + k] = r[k];
+        im[j / 2 * R + k] = i[k];
       }
     }
   }
@@ -279,14 +266,8 @@ struct RegPass {
     float r0, r1, i0, i1;
     f2u(re.v, r0, r1);
     f2u(im.v, i0, i1);
-    const uint32_t a = sm100::pack_half2(r0, i0), b = sm100::pack_half2(r1, i1);
-    if constexpr (R == 32) {
-      w[0][2 * p] = a;
-      w[0][2 * p + 1] = b;
-    } else {
-      w[2 * (p / R)][p % R] = a;
-      w[2 * (p / R) + 1][p % R] = b;
-    }
+    w[2 * (p / R)][p % R] = sm100::pack_half2(r0, i0);
+    w[2 * (p / R) + 1][p % R] = sm100::pack_half2(r1, i1);
   }
 
   template <class A>
@@ -353,11 +334,11 @@ struct RegPass {
       constexpr float sc = 1.f / R1;
 #pragma unroll
       for (int p = 0; p < 16; ++p) {
-        if (R1 < 32 && p % R1 == 0) {
+        if (p % R1 == 0) {
           re[p] = re[p] * num<P2>(sc);
           im[p] = im[p] * num<P2>(sc);
         } else {
-          const float4 f = lds128f(tw + (R1 == 32 ? p : p % R1) * (NV * 16));
+          const float4 f = lds128f(tw + p % R1 * (NV * 16));
           cmulv(re[p], im[p], pack2(f.x, f.y), pack2(f.z, f.w));
         }
         words<R1>(p, re[p], im[p], w);
@@ -395,23 +376,15 @@ struct RegPass {
       if constexpr (POST) {
         // W_N^((k1 + R1 k2) g) / R2: the first factor of each pair and its
         // step, advanced by an FP32 recurrence of 15 steps at most.
-        P2 wr[V2 < 2 ? 1 : V2 / 2], wi[V2 < 2 ? 1 : V2 / 2], sr[V2 < 2 ? 1 : V2 / 2], si[V2 < 2 ? 1 : V2 / 2];
+        P2 wr[V2 / 2], wi[V2 / 2], sr[V2 / 2], si[V2 / 2];
 #pragma unroll
-        for (int q = 0; q < (V2 < 2 ? 1 : V2 / 2); ++q) {
+        for (int q = 0; q < V2 / 2; ++q) {
           float2 f[2], s[2];
-          if constexpr (R2 == 32) {
-            const uint64_t g = (uint64_t)(cb * C + c[0]);
-            f[0] = post_fast(a, k1[0] * g);
-            const float2 st = post_fast(a, (uint64_t)R1 * g);
-            f[1] = cmulf(f[0], st);
-            s[0] = s[1] = cmulf(st, st);
-          } else {
 #pragma unroll
-            for (int u = 0; u < 2; ++u) {
-              const uint64_t g = (uint64_t)(cb * C + c[2 * q + u]);
-              f[u] = post_fast(a, k1[2 * q + u] * g);
-              s[u] = post_fast(a, (uint64_t)R1 * g);
-            }
+          for (int u = 0; u < 2; ++u) {
+            const uint64_t g = (uint64_t)(cb * C + c[2 * q + u]);
+            f[u] = post_fast(a, k1[2 * q + u] * g);
+            s[u] = post_fast(a, (uint64_t)R1 * g);
           }
           wr[q] = pack2(f[0].x * sc, f[1].x * sc);
           wi[q] = pack2(f[0].y * sc, f[1].y * sc);
@@ -420,10 +393,9 @@ struct RegPass {
         }
 #pragma unroll
         for (int p = 0; p < 16; ++p) {
-          constexpr int RR = R2 == 32 ? 16 : R2;
-          const int q = p / RR;
+          const int q = p / R2;
           cmulv(re[p], im[p], wr[q], wi[q]);
-          if (p % RR != RR - 1) cmulv(wr[q], wi[q], sr[q], si[q]);
+          if (p % R2 != R2 - 1) cmulv(wr[q], wi[q], sr[q], si[q]);
           words<R2>(p, re[p], im[p], w);
         }
       } else {

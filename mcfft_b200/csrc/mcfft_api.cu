@@ -542,7 +542,7 @@ mcfftResult add_tile_pass(mcfftPlan p, const PassSpec& s, int only_tile_points =
         tp.tw[dir] = tw;
         continue;
       }
-      const cudaError_t e = gen_reg_twiddles(tw, k->L, k->L / k->R, k->tw_mode, dir == 0 ? -1 : 1,
+      const cudaError_t e = gen_reg_twiddles(tw, k->L, k->L / k->R, k->tw_doubled, dir == 0 ? -1 : 1,
                                              p->split ? 1.0 : 1.0 / k->R, 0);
       if (e != cudaSuccess) return cuda_fail(e);
       tp.tw[dir] = tw;

@@ -10,21 +10,15 @@ constexpr int reg_kind_of(layout::Kind ik, layout::Kind ok) {
   return ik == layout::ROW ? (ok == layout::ROW ? reg::kRR : reg::kRC) : (ok == layout::COL ? reg::kCC : -1);
 }
 
-__global__ void k_gen_reg_twiddles(float* dst, int L, int NV, int mode, int sign, double scale) {
+__global__ void k_gen_reg_twiddles(float* dst, int L, int NV, bool doubled, int sign, double scale) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int R1 = L / NV, n = mode == 2 ? L / 2 : L;
-  if (i >= n) return;
+  if (i >= L) return;
   const int v = i % NV, k = i / NV;
-  float c[2], s[2];
-  for (int u = 0; u < 2; ++u) {
-    const int kk = mode == 2 ? 2 * k + u : k;
-    double ds, dc;
-    sincospi(2.0 * (double)((kk % R1) * v) / (double)L, &ds, &dc);
-    c[u] = (float)(scale * dc);
-    s[u] = (float)(scale * sign * ds);
-  }
-  if (mode == 0) reinterpret_cast<float2*>(dst)[i] = make_float2(c[0], s[0]);
-  else reinterpret_cast<float4*>(dst)[i] = make_float4(c[0], c[1], s[0], s[1]);
+  double ds, dc;
+  sincospi(2.0 * (double)(k * v) / (double)L, &ds, &dc);
+  const float c = (float)(scale * dc), s = (float)(scale * sign * ds);
+  if (doubled) reinterpret_cast<float4*>(dst)[i] = make_float4(c, c, s, s);
+  else reinterpret_cast<float2*>(dst)[i] = make_float2(c, s);
 }
 
 }  // namespace
@@ -53,10 +47,10 @@ bool reg_gather_staging(const TileKernel& k, bool out, int elem, const std::vect
   return reg_gather_staging(RegShape{k.L, k.R, k.C, k.reg_h, k.mma}, out, elem, offs, st, tab);
 }
 
-cudaError_t gen_reg_twiddles(void* dst, int L, int NV, int mode, int sign, double scale,
+cudaError_t gen_reg_twiddles(void* dst, int L, int NV, bool doubled, int sign, double scale,
                              cudaStream_t st) {
-  const int n = mode == 2 ? L / 2 : L, threads = 256;
-  k_gen_reg_twiddles<<<(n + threads - 1) / threads, threads, 0, st>>>(static_cast<float*>(dst), L, NV, mode,
+  const int threads = 256;
+  k_gen_reg_twiddles<<<(L + threads - 1) / threads, threads, 0, st>>>(static_cast<float*>(dst), L, NV, doubled,
                                                                       sign, scale);
   return cudaGetLastError();
 }

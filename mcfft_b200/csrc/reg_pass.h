@@ -28,10 +28,9 @@ void reg_stagings(const TileKernel& k, layout::Kind ik, layout::Kind ok, int in_
 bool reg_gather_staging(const TileKernel& k, bool out, int elem, const std::vector<int64_t>& offs,
                         layout::Staging* st, std::vector<int32_t>* tab);
 
-// Phase-1 twiddles W_L^(k v) * scale in the layout of RegPass (mode 0: FP32,
-// 8 bytes at k NV + v; 1: doubled for two columns, 16 bytes; 2: pairs (2i,
-// 2i + 1), 16 bytes at i NV + v); sign -1 forward, +1 inverse.
-cudaError_t gen_reg_twiddles(void* dst, int L, int NV, int mode, int sign, double scale,
+// Phase-1 twiddles W_L^(k v) * scale in the layout of RegPass (at k NV + v: 8
+// bytes, or doubled for two columns, 16 bytes); sign -1 forward, +1 inverse.
+cudaError_t gen_reg_twiddles(void* dst, int L, int NV, bool doubled, int sign, double scale,
                              cudaStream_t st);
 
 // The kernels without TMA of a 4096-point row tile.
@@ -56,7 +55,7 @@ TileKernel make_reg() {
   k.reg_h = P::h;
   k.tw_bytes = P::TWB;
   k.tab_bytes = P::TABB;
-  k.tw_mode = P::PK ? (R1 == 32 ? 2 : 1) : 0;
+  k.tw_doubled = P::PK;
   add_small<P, Q>(&k);
   return k;
 }

@@ -26,7 +26,8 @@ struct TileKernel {
   int reg_kind = -1;
   const void* fn_inv = nullptr;
   int reg_h = 0;
-  int tw_bytes = 0, tw_mode = 0;
+  int tw_bytes = 0;
+  bool tw_doubled = false;
   int tab_bytes = 0;  // all shared-memory tables of the variant
   // Tensor-core register kernels (fft_mma.cuh): host functions that fill the
   // twiddle table and the matrix fragments of each direction.
