@@ -3,7 +3,7 @@
 Default workload (the configuration the headline metric is quoted on):
 1D forward C2C FFT, N = 2^20, batch 64, FP16 interleaved complex input
 (re/im uniform in [-1, 1), seed 1), plain FP16 form with per-stage 1/16
-scaling.  The split hi+lo form (same FP16 input, FP32 output) is measured
+scaling.  The split form (same FP16 input, FP32 output) is measured
 on the same data and reported under "split", the uneven batch under
 "uneven_batch".
 
@@ -413,8 +413,7 @@ def run_ours(args, rank, world, local_rank):
 
     result = None
     if rank == 0:
-        split_form = ("FP16 input split hi+lo, FP32 output" if s16 else
-                      "FP32 input split hi+lo, FP32 output")
+        split_form = f"{'FP16' if s16 else 'FP32'} input, FP32 arithmetic and output"
         result = {
             "metric": METRIC,
             "value": round(value, 2),

@@ -15,10 +15,14 @@
 // vectors -- the packed FP32x2 operand of the twiddle product.  tcgen05 would
 // need its operand staged in shared memory and its result read back from
 // tensor memory: eight shared-memory crossings per tile instead of six, for a
-// contraction of only 32 x 32; the FP32 register form (RegPass) needs 36 to
-// 43 cycles of the FP32 pipe per point and sub-partition against about 46
-// that the copies of a tile take, this form 10 to 25 there beside 16 on the
-// tensor pipe (a warp-wide m16n8k16 takes eight cycles of a sub-partition).
+// contraction of only 32 x 32.
+//
+// What bounds it: the copies, then the serial chain of a tile's phases.  2^20 x
+// 64, counters of both passes: a sub-partition spends 14 and 26 cycles of the
+// FP32 pipe on 32 points (two per packed instruction; the FP32 register form,
+// RegPass, 31 and 40), 16 of the tensor pipe (eight per warp-wide m16n8k16)
+// and 16 and 29 issue slots, where the copies of the tile alone take about 52.
+// Both passes together 213 us, the copies alone 194.
 //
 // Every shared access moves 16 bytes: a thread's 32 points are eight chunks
 // of four, and which digit runs within a chunk, along the lanes and along the

@@ -12,7 +12,7 @@
 // FP32) tile is 64 KB in and 64 KB out, 5.9 K cycles of one SM's share of the
 // copy bandwidth.  The tile crosses shared memory six times (TMA in, phase 1
 // load and store, phase 2 load and store, TMA out): 3 K wavefronts of 128
-// bytes plus 0.3 .. 1 K of twiddles, and about 3 K cycles of the FP32 pipe.
+// bytes plus 0.6 .. 0.9 K of twiddles, and 2 to 2.6 K cycles of the FP32 pipe.
 // The tcgen05 form of the same pass (fft_tile.cuh) crosses it eight times and
 // reads its stage operands and twiddle rows on top, 5.6 K wavefronts in
 // phases that wait for one another; a 16-point DFT as a real 32 x 32 product

@@ -391,9 +391,15 @@ bool gather_rows(const layout::Staging& tile_st, int64_t L, int64_t C,
 // against 8.2 us, 256 x 1000 4.1 / 7.5, 64 x 5000 4.1 / 8.2, 512 x 5000 8.2 /
 // 10.3, 512 x 9001 14.3 / 14.3.  Past about four full tiles per SM the two
 // tie, and as the first pass of a 2D transform the full tiles are faster
-// (1024^2 x 16: 57.4 against 59.4 us).
+// (1024^2 x 16: 57.4 against 59.4 us).  Split form, 4096-point tiles (up to six
+// per SM without TMA) against full ones of 8K points, FP32 / FP16 input: 512 x
+// 600 4.1 / 4.1 against 8.2 / 6.2, 512 x 7000 12.3 / 12.3 against 12.3 / 10.3,
+// 512 x 12500 18.6 / 14.4 against 22.5 / 16.4, 512 x 18000 (the line) 26.8 /
+// 22.8 against 28.8 / 24.6, 64 x 140000 26.5 / 19.5 against 27.1 / 22.6.
 bool small_tiles(const mcfftPlan p, const PassSpec& s) {
-  if (s.L == 4096) return true;  // the register kernel of this length has one tile size
+  // The 16K-point routine of this length belongs to the one-launch kernel;
+  // split: 256 transforms 6.2 us, 16384 168, on the tcgen05 tiles 12.4 and 424.
+  if (s.L == 4096) return true;
   return s.in_sp == 1 && s.out_sp == 1 && s.L * s.ncols * s.nouter <= int64_t(4) * p->sms * 16384;
 }
 
@@ -441,8 +447,13 @@ mcfftResult add_tile_pass(mcfftPlan p, const PassSpec& s, int only_tile_points =
   std::vector<int32_t> in_tab, out_tab;
   const bool indexed = s.gather || !s.in_idx.empty() || !s.out_idx.empty();
   // Register kernels (fft_reg.cuh, fft_mma.cuh, fft_rows.cuh) first: faster
-  // than the tcgen05 tiles in every case measured (split form 1.33x .. 1.39x
-  // on four-step, 2D and 3D transforms, plain 1.04x .. 1.13x).  Passes of the
+  // than the tcgen05 tiles (split form 1.3x .. 1.4x on four-step, 2D and 3D
+  // transforms, plain 1.1x on 2^20 x 64, 1.25x .. 1.3x on 2D and 3D, rows of
+  // few points 1.5x .. 2x).  One exception is known: plain pairs of passes of
+  // at most 2^18 points in all (sixteen 16K-point tiles) take 14.4 us, with
+  // both passes on 8K-point tcgen05 tiles 12.3, which the plan-time tuner does
+  // not see, as it times a pass by itself; those tiles round more often (error
+  // 7.6e-4 against 4.8e-4), so nothing forces them.  Passes of the
   // batch queue, longer columns and the plain form's 8K-point tiles (small
   // batches) take the tcgen05 tiles; those of the one-launch kernel are
   // register passes or none.  A size that MCFFT_TILE_POINTS names is the only
