@@ -171,7 +171,9 @@ class Plan:
         # refuses those (TypeError)
         if not (type(in_ptr) is int and type(out_ptr) is int and type(stream) is int):
             in_ptr, out_ptr, stream = (ctypes.c_void_p(v) for v in (in_ptr, out_ptr, stream))
-        _check(lib().mcfftExec(self._h, in_ptr, out_ptr, direction, stream), "mcfftExec")
+        rc = (_lib or lib()).mcfftExec(self._h, in_ptr, out_ptr, direction, stream)
+        if rc != SUCCESS:
+            raise McfftError(rc, "mcfftExec")
 
     def exec_host_ptr(self, in_ptr: int, out_ptr: int, direction: int = FORWARD, stream: int = 0):
         """Host buffers in and out (page-locked for overlapped copies): copy
